@@ -84,6 +84,7 @@ constexpr int pair_minb() {
 #ifndef SOFIA_SEARCH_ZWIN
 #define SOFIA_SEARCH_ZWIN 1
 #endif
+constexpr int ESLOT = 4;  // energy partial sums per list row (see pair_body)
 constexpr int FLUSH = SOFIA_PAIR_FLUSH;  // list entries between FP32 -> fixed-point flushes of the i forces
 static_assert(FLUSH >= 1 && FLUSH <= 32 && (32 % FLUSH) == 0, "FLUSH must divide 32");
 
@@ -881,7 +882,12 @@ __device__ __forceinline__ void flush_i(long long *__restrict__ fi, int lane, T 
 // Integer addition makes every sum independent of the order of the atomics, so
 // results stay bit-reproducible.  EN adds the LJ and Coulomb energies, VIR the
 // diagonal virial (each pair once).
-template <typename T, bool EN, bool VIR, bool SAME, bool TRI>
+//
+// SPLIT warps share a row: warp `part` takes the 32-entry batches part, part +
+// SPLIT, ... of it.  A batch is flushed to fixed point as a whole either way, so
+// forces do not depend on SPLIT; energies are kept as ESLOT partial sums per row,
+// batch b adding to slot b % ESLOT in batch order, so they do not either.
+template <typename T, bool EN, bool VIR, bool SAME, bool TRI, int SPLIT>
 __device__ __forceinline__ void pair_body(
     int bx, int maxcl, const int *__restrict__ ncl_dev, const AtomRec *__restrict__ rec,
     const int *__restrict__ jlist, const unsigned long long *__restrict__ jmask,
@@ -932,7 +938,9 @@ __device__ __forceinline__ void pair_body(
     for (int c = 0; c < 6; ++c) fi[c * 32 + lane] = 0;
     __syncthreads();
     const int jj = lane & 7, q = lane >> 3;
-    const int icl = (bx * blockDim.x + threadIdx.x) >> 5;
+    static_assert(ESLOT % SPLIT == 0, "an energy slot belongs to one warp of the row");
+    const int wid = (bx * blockDim.x + threadIdx.x) >> 5;
+    const int icl = wid / SPLIT, part = wid % SPLIT;
     if (icl >= maxcl || icl >= ncl_dev[0]) return;
     const size_t stride = (size_t)maxcl * CL;
     // this lane's share of the reduced j force: component q (3 = none) of j atom jj
@@ -952,7 +960,7 @@ __device__ __forceinline__ void pair_body(
     float2 ax2 = z2, ay2 = z2, az2 = z2, alj2 = z2, ac2 = z2, axx2 = z2, ayy2 = z2, azz2 = z2;
     const float2 qiq2 = make_float2((float)qiq0, (float)qiq1);
     double e_lj = 0.0, e_c = 0.0, vxx = 0.0, vyy = 0.0, vzz = 0.0;
-    for (int base = 0; base < n; base += 32) {
+    for (int base = 32 * part; base < n; base += 32 * SPLIT) {
         const int cnt = min(32, n - base);
         const int myw = (lane < cnt) ? row[base + lane] : 0;
         const unsigned long long mym = (lane < cnt) ? mrow[base + lane] : 0ull;
@@ -1135,6 +1143,27 @@ __device__ __forceinline__ void pair_body(
                 }
             }
         }
+        if (EN || VIR) {
+            // the batch's sums over the warp, added to its energy slot of the row
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                e_lj += __shfl_xor_sync(FULL, e_lj, off);
+                e_c += __shfl_xor_sync(FULL, e_c, off);
+                if (VIR) {
+                    vxx += __shfl_xor_sync(FULL, vxx, off);
+                    vyy += __shfl_xor_sync(FULL, vyy, off);
+                    vzz += __shfl_xor_sync(FULL, vzz, off);
+                }
+            }
+            const int b = base >> 5;
+            if (lane < 5) {
+                double *o = energy + ((size_t)icl * ESLOT + b % ESLOT) * 5 + lane;
+                const double v = lane == 0 ? e_lj : lane == 1 ? e_c : lane == 2 ? vxx
+                               : lane == 3 ? vyy : vzz;
+                o[0] = b < ESLOT ? v : o[0] + v;
+            }
+            e_lj = e_c = vxx = vyy = vzz = 0.0;
+        }
     }
     // sum each i atom's partials over its 8 lanes (lane bits 0-2), then lane
     // jj = 0 of each quarter adds the totals of i atoms q and q + 4
@@ -1156,37 +1185,20 @@ __device__ __forceinline__ void pair_body(
         }
     }
     if (EN || VIR) {
-        e_lj += (double)a_lj;
-        e_c += (double)a_c;
-        vxx += (double)a_xx;
-        vyy += (double)a_yy;
-        vzz += (double)a_zz;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            e_lj += __shfl_xor_sync(FULL, e_lj, off);
-            e_c += __shfl_xor_sync(FULL, e_c, off);
-            vxx += __shfl_xor_sync(FULL, vxx, off);
-            vyy += __shfl_xor_sync(FULL, vyy, off);
-            vzz += __shfl_xor_sync(FULL, vzz, off);
-        }
-        if (lane == 0) {
-            double *o = energy + (size_t)icl * 5;
-            o[0] = e_lj;
-            o[1] = e_c;
-            o[2] = vxx;
-            o[3] = vyy;
-            o[4] = vzz;
-        }
+        // slots past the row's batches
+        for (int b = (n + 31) >> 5; b < ESLOT; ++b)
+            if (b % SPLIT == part && lane < 5)
+                energy[((size_t)icl * ESLOT + b) * 5 + lane] = 0.0;
     }
 }
-template <typename T, bool EN, bool VIR, bool SAME, bool TRI = false>
+template <typename T, bool EN, bool VIR, bool SAME, bool TRI = false, int SPLIT = 1>
 __global__ void __launch_bounds__((pair_block<T, EN>()), (pair_minb<T, EN>())) k_pair(
     int maxcl, const int *__restrict__ ncl_dev, const AtomRec *__restrict__ rec,
     const int *__restrict__ jlist, const unsigned long long *__restrict__ jmask,
     const int *__restrict__ jcount, int jcap, const float4 *__restrict__ ljtab, PairConst k,
     unsigned long long *__restrict__ fslot, double *__restrict__ energy) {
     SOFIA_PDL_ENTRY();
-    pair_body<T, EN, VIR, SAME, TRI>(blockIdx.x, maxcl, ncl_dev, rec, jlist, jmask, jcount, jcap,
+    pair_body<T, EN, VIR, SAME, TRI, SPLIT>(blockIdx.x, maxcl, ncl_dev, rec, jlist, jmask, jcount, jcap,
                                 ljtab, k, k.L, fslot, energy);
 }
 
@@ -1425,10 +1437,11 @@ __global__ void k_set_flag(int *__restrict__ flag, int v) {
 
 // Two-stage deterministic column sums: stage 1 = fixed grid of blocks over
 // contiguous ranges (coalesced), stage 2 = one block over the partials.
+// n rows at most, ESLOT per cluster of ncl_dev.
 __device__ __forceinline__ void red_stage1_body(int bx, int n, int w, const int *__restrict__ ncl_dev,
                              const double *__restrict__ in, double *__restrict__ part, int nblk) {
     __shared__ double s[256];
-    const int nn = ncl_dev ? min(n, ncl_dev[0]) : n;
+    const int nn = min(n, ncl_dev[0] * ESLOT);
     const int chunk = (nn + nblk - 1) / nblk;
     const int b0 = bx * chunk, b1 = min(nn, b0 + chunk);
     for (int c = 0; c < w; ++c) {
@@ -1537,7 +1550,7 @@ static int sys_alloc(Sys *s) {
     SOFIA_CUDA(ctx, s->bb.ensure(sizeof(float4) * 2 * maxcl));
     SOFIA_CUDA(ctx, s->jcount.ensure(sizeof(int) * maxcl));
     SOFIA_CUDA(ctx, s->nclusters.ensure(sizeof(int) * 4));
-    SOFIA_CUDA(ctx, s->energy.ensure(sizeof(double) * 5 * maxcl));
+    SOFIA_CUDA(ctx, s->energy.ensure(sizeof(double) * 5 * ESLOT * maxcl));
     SOFIA_CUDA(ctx, s->red.ensure(sizeof(double) * 8));
     SOFIA_CUDA(ctx, s->flag.ensure(sizeof(int) * 4));
     SOFIA_CUDA(ctx, s->status_local.ensure(sizeof(int) * ST_NSLOTS));
@@ -1832,54 +1845,86 @@ int sys_eval(Sys *s, int precision, bool energy, bool virial, bool force_build) 
     return sys_pair(s, precision, energy, virial);
 }
 
+// Warps per list row of the pair kernels.  A row of about 70 entries is one
+// serial chain per warp (45 us at 9,000 atoms, whose 1,175 rows are a quarter of
+// the warps the GPU can hold), so a system whose rows leave warps idle gives
+// each row 2 or 4 of them; every extra warp repeats the row's prologue and its
+// i-force reduction, so rows that fill the GPU keep one.  Mixed: 4 while 4 warps
+// per row are resident at once, 2 while the rows are (MD us per step at 1 / 2 / 4:
+// 3,000 atoms 71 / 60 / 53, 9,000 92 / 73 / 62, 12,000 - / 73 / 76, 16,000 93 / 78 /
+// 80, 37,000 125 / 123 / 134, 275,000 605 / 626 / 750).  FP64 runs half as many warps
+// and is bound by its pipe sooner: 2 only while both fit (3,000 atoms 116 / 89 / -,
+// 9,000 128 / 100 / 127, 16,000 140 / 143 / -).
+static int pair_split(const Sys *s, int precision) {
+    // the table of this many types allows one block less per SM: one warp per row
+    if (pair_smem(s->ntypes, false, true) > 32768) return 1;
+    const bool mixed = precision != SOFIA_PREC_FP64;
+    // resident warps, and the rows (half of a column's last cluster is empty on average)
+    const long res = (long)s->nsm * (mixed ? 32 : 16);
+    const long rows = s->n / CL + s->ncols / 2;
+    if (4 * rows <= res) return 4;
+    return (mixed ? rows : 2 * rows) <= res ? 2 : 1;
+}
+
+template <typename T, bool EN, bool VIR, bool TRI, int SPLIT>
+static void launch_pair_one(Sys *s, const PairConst &k) {
+    const int block = pair_block<T, EN>();
+    launch_pdl(k_pair<T, EN, VIR, true, TRI, SPLIT>,
+               grid_for((long)s->max_clusters * SPLIT * 32, block), block,
+               pair_smem(s->ntypes, TRI, EN), s->ctx->stream, s->max_clusters,
+               s->nclusters.as<int>(), s->rec.as<AtomRec>(), s->ilist.as<int>(),
+               s->imask.as<unsigned long long>(), s->icount.as<int>(), s->jcap,
+               s->ljtab.as<float4>(), k, s->fslot.as<unsigned long long>(),
+               s->energy.as<double>());
+}
+
+template <int SPLIT>
+static void launch_pair(Sys *s, int precision, bool energy, bool virial, const PairConst &k) {
+    // the blocks of a shared row do too little work to fill the three-index table
+    const bool tri = (energy || virial) && pair_tri(s->ntypes) && SPLIT == 1;
+    if (precision == SOFIA_PREC_FP64) {
+        if (virial)
+            launch_pair_one<double, true, true, false, SPLIT>(s, k);
+        else if (energy)
+            launch_pair_one<double, true, false, false, SPLIT>(s, k);
+        else
+            launch_pair_one<double, false, false, false, SPLIT>(s, k);
+    } else if (tri) {
+        if (virial)
+            launch_pair_one<float, true, true, SPLIT == 1, SPLIT>(s, k);
+        else
+            launch_pair_one<float, true, false, SPLIT == 1, SPLIT>(s, k);
+    } else if (virial) {
+        launch_pair_one<float, true, true, false, SPLIT>(s, k);
+    } else if (energy) {
+        launch_pair_one<float, true, false, false, SPLIT>(s, k);
+    } else {
+        launch_pair_one<float, false, false, false, SPLIT>(s, k);
+    }
+}
+
 // Pair kernel (+ energy reduction) on the pruned list.
 int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
              const LangevinArgs *lg, float *ff_out) {
     sofia_nb_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     PairConst k = make_pair_const(s, nullptr);
-    // blocks of the force-only FP32 kernel and of the others (energies, FP64)
-    const int blocks = grid_for((long)s->max_clusters * 32, SOFIA_PAIR_BLOCK);
-    const int blocks_en = grid_for((long)s->max_clusters * 32, SOFIA_PAIR_BLOCK_EN);
-    const size_t smem = pair_smem(s->ntypes, false, energy || virial);
-    const bool tri = (energy || virial) && pair_tri(s->ntypes);
-    const size_t smem3 = pair_smem(s->ntypes, tri, energy || virial);
-    long long *fx = s->f[0].as<long long>(), *fy = s->f[1].as<long long>(),
-              *fz = s->f[2].as<long long>();
-#define SOFIA_PAIR_ARGS                                                                   \
-    s->max_clusters, s->nclusters.as<int>(), s->rec.as<AtomRec>(), s->ilist.as<int>(),    \
-        s->imask.as<unsigned long long>(), s->icount.as<int>(), s->jcap,                  \
-        s->ljtab.as<float4>(), k, s->fslot.as<unsigned long long>(), s->energy.as<double>()
+    const int split = pair_split(s, precision);
     if (s->timing) cudaEventRecord(s->ev[2], st);
     // sofia_system_create requires rcut == cut_coul: one cut-off gates both terms
-    if (precision == SOFIA_PREC_FP64) {
-        if (virial)
-            sofia::launch_pdl(k_pair<double, true, true, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem, st, SOFIA_PAIR_ARGS);
-        else if (energy)
-            sofia::launch_pdl(k_pair<double, true, false, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem, st, SOFIA_PAIR_ARGS);
-        else
-            sofia::launch_pdl(k_pair<double, false, false, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem, st, SOFIA_PAIR_ARGS);
-    } else if (tri) {
-        if (virial)
-            sofia::launch_pdl(k_pair<float, true, true, true, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem3, st,
-                              SOFIA_PAIR_ARGS);
-        else
-            sofia::launch_pdl(k_pair<float, true, false, true, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem3, st,
-                              SOFIA_PAIR_ARGS);
-    } else {
-        if (virial)
-            sofia::launch_pdl(k_pair<float, true, true, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem, st, SOFIA_PAIR_ARGS);
-        else if (energy)
-            sofia::launch_pdl(k_pair<float, true, false, true>, blocks_en, SOFIA_PAIR_BLOCK_EN, smem, st, SOFIA_PAIR_ARGS);
-        else
-            sofia::launch_pdl(k_pair<float, false, false, true>, blocks, SOFIA_PAIR_BLOCK, smem, st, SOFIA_PAIR_ARGS);
-    }
-#undef SOFIA_PAIR_ARGS
+    if (split == 4)
+        launch_pair<4>(s, precision, energy, virial, k);
+    else if (split == 2)
+        launch_pair<2>(s, precision, energy, virial, k);
+    else
+        launch_pair<1>(s, precision, energy, virial, k);
     if (s->timing) {
         cudaEventRecord(s->ev[3], st);
         s->pending_pair = 1;
     }
     const int nslots = s->max_clusters * CL;
+    long long *fx = s->f[0].as<long long>(), *fy = s->f[1].as<long long>(),
+              *fz = s->f[2].as<long long>();
     LangevinArgs lgv{};
     if (lg) lgv = *lg;
     sofia::launch_pdl(k_unpack, grid_for(nslots, 256), 256, 0, st, nslots, s->nclusters.as<int>(),
@@ -1889,7 +1934,7 @@ int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
                                                     s->dcount.as<long long>(), lgv, ff_out);
     s->launches += 2;
     if (energy || virial) {
-        sofia::launch_pdl(k_red_stage1, RED_BLOCKS, 256, 0, st, s->max_clusters, 5, s->nclusters.as<int>(),
+        sofia::launch_pdl(k_red_stage1, RED_BLOCKS, 256, 0, st, s->max_clusters * ESLOT, 5, s->nclusters.as<int>(),
                                                  s->energy.as<double>(), s->part.as<double>());
         // the half list holds each pair once: no halving
         sofia::launch_pdl(k_red_stage2, 1, 256, 0, st, RED_BLOCKS, 5, s->part.as<double>(), s->red.as<double>(),
@@ -2003,9 +2048,12 @@ extern "C" int sofia_system_create(sofia_nb_ctx *ctx, const sofia_system_desc *d
         return sofia::fail(ctx, SOFIA_EINVAL, "the cluster path needs rcut == cut_coul%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
     SOFIA_CUDA(ctx, sofia::pair_smem_optin(d->ntypes));
+    int nsm = 0;
+    SOFIA_CUDA(ctx, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     sofia_system *ss = new sofia_system();
     Sys *s = &ss->s;
     s->ctx = ctx;
+    s->nsm = nsm;
     s->n = d->np;
     s->ntypes = d->ntypes;
     s->precision = d->precision;
@@ -2534,7 +2582,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4) ? (EN ? SOFIA_PAIR_MINB_
     k_pair_b(BatchDev *__restrict__ tab, PairConst k) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_W256)
-    pair_body<T, EN, VIR, SAME, TRI>(lb, d.maxcl, d.ncl, d.rec, d.ilist, d.imask, d.icount, d.jcap,
+    pair_body<T, EN, VIR, SAME, TRI, 1>(lb, d.maxcl, d.ncl, d.rec, d.ilist, d.imask, d.icount, d.jcap,
                                 d.ljtab, k, d.L, d.fslot, d.energy);
     __syncthreads();
     SOFIA_BATCH_END
@@ -2551,7 +2599,7 @@ __global__ void __launch_bounds__(256, SOFIA_BATCH_STREAM_MINB) k_unpack_b(const
 __global__ void k_red_stage1_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_RED)
-    red_stage1_body(lb, d.maxcl, 5, d.ncl, d.energy, d.part, RED_BLOCKS);
+    red_stage1_body(lb, d.maxcl * ESLOT, 5, d.ncl, d.energy, d.part, RED_BLOCKS);
     __syncthreads();
     SOFIA_BATCH_END
 }

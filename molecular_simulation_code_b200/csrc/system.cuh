@@ -68,6 +68,7 @@ struct Md {
 struct Sys {
     sofia_nb_ctx *ctx = nullptr;
     int n = 0, ntypes = 0, precision = 0;
+    int nsm = 148;                    // multiprocessors of the device
     double L = 0.0;
     float box = 0.0f;
     double alpha = 0.0, rc = 0.0, rlist = 0.0, skin = 0.0, e_shift = 0.0, f_shift = 0.0;
@@ -89,7 +90,7 @@ struct Sys {
     DevBuf sref;                        // build-time data in slot order (see pack_body)
     DevBuf atom_slot;                   // cluster slot of every atom (inverse of slot_orig)
     DevBuf status_local;
-    DevBuf energy;                      // per-i-cluster energy partials (pot, ecoul, vir x,y,z)
+    DevBuf energy;                      // energy partials per i-cluster and slot (pot, ecoul, vir x,y,z)
     DevBuf red;                         // reduced energies
     DevBuf flag;                        // rebuild flag (int)
     DevBuf stage_pos, stage_ff;
