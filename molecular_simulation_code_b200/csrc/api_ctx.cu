@@ -44,10 +44,11 @@ extern "C" int sofia_nb_destroy(sofia_nb_ctx *ctx) {
     ctx->cell_of.release();
     ctx->cell_count.release();
     ctx->cell_start.release();
-    ctx->cell_fill.release();
+    ctx->cell_rank.release();
     ctx->sorted_idx.release();
     ctx->pos_sorted.release();
-    ctx->cnum.release();
+    ctx->pos_pair.release();
+    ctx->slot_of.release();
     ctx->pe_atom.release();
     ctx->red_out.release();
     ctx->res_nlist.release();

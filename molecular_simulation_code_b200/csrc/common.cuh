@@ -48,6 +48,7 @@ enum StatusSlot {
     ST_NCLUSTER = 8,     // cluster-pair list fill
     ST_FIXED_OVF = 9,    // fixed-point force range exceeded
     ST_SHAKE_NC = 10,    // SHAKE groups that hit maxiter (warning, as the reference prints)
+    ST_UNWRAPPED = 11,   // a coordinate outside [0, box] was binned
     ST_NSLOTS = 16
 };
 
@@ -80,7 +81,8 @@ struct sofia_nb_ctx {
     // staging buffers for host-pointer arguments
     sofia::DevBuf stage[12];
     // reference-semantics cell grid / list scratch
-    sofia::DevBuf cell_of, cell_count, cell_start, cell_fill, sorted_idx, pos_sorted, cnum;
+    sofia::DevBuf cell_of, cell_count, cell_start, cell_rank, sorted_idx, pos_sorted, pos_pair,
+        slot_of;
     sofia::DevBuf pe_atom;   // per-atom energy partials
     sofia::DevBuf red_out;   // reduction output
     // resident reference list (kept when the caller passes nlist == NULL to the force call)

@@ -11,6 +11,7 @@
 // candidate sweep, neighbour rows of neigh_alloc int32 per atom (Fortran
 // nlist(neigh_alloc*(i-1)+j)).
 #include <climits>
+#include <cmath>
 #include <mutex>
 
 #include "common.cuh"
@@ -33,9 +34,19 @@ __device__ __forceinline__ int bin_axis(float x, double boxd, double irn, int D,
     return ix;
 }
 
+// Clears the cell counts and the status words of a build.
+__global__ void k_clear_cells(int n, int *__restrict__ cell_count, int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) cell_count[i] = 0;
+    if (i < sofia::ST_NSLOTS) status[i] = 0;
+}
+
+// Cell of every atom and its arrival rank in the cell.
 __global__ void k_bin_atoms(int np, const float4 *__restrict__ pos, double boxd, double irn,
-                            int D, int *__restrict__ cell_of, int *__restrict__ cell_count,
-                            int *__restrict__ status) {
+                            int D, int *__restrict__ cell_of, int *__restrict__ rank,
+                            int *__restrict__ cell_count, int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
     float4 p = pos[i];
@@ -45,55 +56,109 @@ __global__ void k_bin_atoms(int np, const float4 *__restrict__ pos, double boxd,
     int iz = bin_axis(p.z, boxd, irn, D, &bad);
     int c = ix + iy * D + iz * D * D;
     cell_of[i] = c;
-    atomicAdd(&cell_count[c], 1);
+    rank[i] = atomicAdd(&cell_count[c], 1);
     if (bad) atomicAdd(&status[sofia::ST_BADBIN], 1);
+    auto inside = [boxd](float x) { return x >= 0.0f && (double)x <= boxd; };
+    if (!(inside(p.x) && inside(p.y) && inside(p.z))) status[sofia::ST_UNWRAPPED] = 1;
 }
 
-// Exclusive scan of n counts into start[0..n] by one block (cells are few).
-__global__ void k_scan_block(int n, const int *__restrict__ in, int *__restrict__ out) {
-    __shared__ int s[1024];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
+constexpr int LIST_ATOMS = 8;  // atoms per warp of the list build
+
+// Exclusive scans by one block (cells are few): of the n cell counts into
+// start[0..n], and of the cells' chunks of LIST_ATOMS atoms into chunk[0..n].
+__global__ void __launch_bounds__(1024) k_scan_block(int n, const int *__restrict__ in,
+                                                     int *__restrict__ start,
+                                                     int *__restrict__ chunk) {
+    SOFIA_PDL_ENTRY();
+    __shared__ int2 s_w[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    int2 carry = make_int2(0, 0);
     for (int base = 0; base < n; base += 1024) {
-        int t = threadIdx.x;
-        int v = (base + t < n) ? in[base + t] : 0;
-        s[t] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            int a = (t >= off) ? s[t - off] : 0;
-            __syncthreads();
-            s[t] += a;
-            __syncthreads();
+        const int v = (base + t < n) ? in[base + t] : 0, u = (v + LIST_ATOMS - 1) / LIST_ATOMS;
+        int2 incl = make_int2(v, u);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int a = __shfl_up_sync(FULL, incl.x, off), b = __shfl_up_sync(FULL, incl.y, off);
+            if (lane >= off) {
+                incl.x += a;
+                incl.y += b;
+            }
         }
-        if (base + t < n) out[base + t] = carry + s[t] - v;
+        if (lane == 31) s_w[w] = incl;
         __syncthreads();
-        if (t == 1023) carry += s[1023];
+        int2 before = make_int2(0, 0), total = make_int2(0, 0);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+            const int2 x = s_w[k];
+            if (k < w) {
+                before.x += x.x;
+                before.y += x.y;
+            }
+            total.x += x.x;
+            total.y += x.y;
+        }
+        if (base + t < n) {
+            start[base + t] = carry.x + before.x + incl.x - v;
+            chunk[base + t] = carry.y + before.y + incl.y - u;
+        }
+        carry.x += total.x;
+        carry.y += total.y;
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[n] = carry;
+    if (t == 0) {
+        start[n] = carry.x;
+        chunk[n] = carry.y;
+    }
 }
 
 __global__ void k_scatter(int np, const int *__restrict__ cell_of, const int *__restrict__ start,
-                          int *__restrict__ fill, int *__restrict__ sorted) {
+                          const int *__restrict__ rank, int *__restrict__ sorted) {
+    SOFIA_PDL_ENTRY();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
-    int c = cell_of[i];
-    int slot = atomicAdd(&fill[c], 1);
-    sorted[start[c] + slot] = i;
+    sorted[start[cell_of[i]] + rank[i]] = i;
 }
 
 // Orders every cell's atoms by input index (ascending, or descending = the
-// reference's head-of-chain order, mod_neighbor.f90:933-941 + :956-980).
-__global__ void k_sort_cells(int ncell, const int *__restrict__ start, int *__restrict__ sorted,
-                             int descending, int *__restrict__ status) {
+// reference's head-of-chain order, mod_neighbor.f90:933-941 + :956-980), then
+// gathers the cell's positions in that order into ps, or for the list build (pair
+// not NULL) as {-x, -y, -z, input index}, with the inverse order in slot_of.  A cell of up to RANK_SORT atoms is ordered
+// by counting, one pass over shared memory per atom; a bitonic sort of 130 atoms
+// takes 36 block barriers instead.
+constexpr int RANK_SORT = 512;
+__global__ void __launch_bounds__(256) k_sort_cells(
+    int ncell, const int *__restrict__ start, int *__restrict__ sorted, int descending,
+    const float4 *__restrict__ pos, float4 *__restrict__ ps, float4 *__restrict__ pair,
+    int *__restrict__ slot_of, int *__restrict__ bin_sorted, int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
     __shared__ int s[MAX_CELL_SORT];
     int c = blockIdx.x;
     if (c >= ncell) return;
     int b = start[c], n = start[c + 1] - b;
-    if (n <= 1) return;
     if (n > MAX_CELL_SORT) {
         if (threadIdx.x == 0) atomicAdd(&status[sofia::ST_CELLOVER], 1);
+        return;
+    }
+    auto place = [&](int at, int i) {
+        sorted[b + at] = i;
+        bin_sorted[b + at] = c;
+        const float4 p = pos[i];
+        if (pair) {
+            pair[b + at] = make_float4(-p.x, -p.y, -p.z, __int_as_float(i));
+            slot_of[i] = b + at;
+        } else {
+            ps[b + at] = p;
+        }
+    };
+    if (n <= RANK_SORT) {
+        for (int t = threadIdx.x; t < n; t += blockDim.x) s[t] = sorted[b + t];
+        __syncthreads();
+        for (int t = threadIdx.x; t < n; t += blockDim.x) {
+            const int v = s[t];
+            int less = 0;
+            for (int k = 0; k < n; ++k) less += s[k] < v;
+            place(descending ? n - 1 - less : less, v);
+        }
         return;
     }
     int m = 1;
@@ -119,99 +184,230 @@ __global__ void k_sort_cells(int ncell, const int *__restrict__ start, int *__re
             __syncthreads();
         }
     }
-    for (int t = threadIdx.x; t < n; t += blockDim.x) sorted[b + t] = descending ? -s[t] : s[t];
+    for (int t = threadIdx.x; t < n; t += blockDim.x) place(t, descending ? -s[t] : s[t]);
 }
 
-__global__ void k_gather_sorted(int np, const int *__restrict__ sorted,
-                                const float4 *__restrict__ pos, const int *__restrict__ cell_of,
-                                float4 *__restrict__ ps, int *__restrict__ bin_sorted) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= np) return;
-    int i = sorted[k];
-    ps[k] = pos[i];
-    bin_sorted[k] = cell_of[i];
-}
+// build_neighbor_nonewton_nomic, mod_neighbor.f90:622-809, over the stencil of
+// neighcell_nonewton (:1309-1378): the own cell, then the 26 others z-major.
+// A warp takes a chunk of 8 atoms of one cell and sweeps the stencil's atoms in
+// order, 32 candidates at a time: they are staged in shared memory, lane (a, q) tests
+// atom a against candidates 8q .. 8q + 7, two per packed FP32x2 operation, and keeps
+// the outcomes as sign bits; the four lanes of an atom combine them to its 32-bit
+// mask, and the warp writes each atom's survivors compacted by that mask, coalesced
+// and in the reference's order.
+//
+// The sweep is bound by instruction issue (about 3,600 candidates per atom at 10.9 A
+// cells, 20 % of them inside the list radius), so what it leaves out per candidate
+// is what it gains:
+//   * stencil cells that follow one another in memory are swept as one run;
+//   * with at least 5 cells per side and every coordinate in [0, box] (the binning
+//     also takes others) the minimum image is the same for a whole stencil cell:
+//     |dx| is at most 2/5 box without a wrap and at least 3/5 box with one, so
+//     rint(dx * ibox) is 0 or the sign of the wrap, and dx - rint() * box is one
+//     addition of +-box, or nothing, with the same rounding;
+//   * (double)dr2 < rv2 is dr2 < lim, the smallest float that is not below rv2, and
+//     that is the sign of dr2 - lim;
+//   * an atom and its partners become a mask over the 32 candidates, made only for
+//     tiles that can hold one of them.
+// 45,255 atoms, 12 A: 224 us (171 M warp instructions); 527 us as one warp per atom
+// with the minimum image and 12 partner compares per candidate, 254 us as one warp per
+// two atoms with a ballot per atom and 32 candidates, 227 us as one atom per lane with
+// a buffer column each (99 M instructions, but 12 warps per SM).
+constexpr int LIST_WARPS = 8;
+struct ListTile {
+    float x[32], y[32], z[32];  // negated coordinates
+};
 
-// neighcell_nonewton, mod_neighbor.f90:1309-1378.
-__global__ void k_stencil(int ncellT, int D, int *__restrict__ cnum) {
-    int ic = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ic >= ncellT) return;
-    int icz = ic / (D * D);
-    int icy = (ic - icz * D * D) / D;
-    int icx = ic - icy * D - icz * D * D;
-    int *out = cnum + 27 * ic;
-    out[0] = ic;
-    int k = 1;
-    for (int iz = -1; iz <= 1; ++iz)
-        for (int iy = -1; iy <= 1; ++iy)
-            for (int ix = -1; ix <= 1; ++ix) {
-                if (iz == 0 && iy == 0 && ix == 0) continue;
-                int zc = icz + iz, yc = icy + iy, xc = icx + ix;
-                zc = zc < 0 ? zc + D : (zc >= D ? zc - D : zc);
-                yc = yc < 0 ? yc + D : (yc >= D ? yc - D : yc);
-                xc = xc < 0 ? xc + D : (xc >= D ? xc - D : xc);
-                out[k++] = xc + yc * D + zc * D * D;
-            }
-}
-
-// build_neighbor_nonewton_nomic, mod_neighbor.f90:622-809.  One warp per atom
-// (taken in cell order so warps in flight share stencils in L1/L2); lanes
-// sweep 32 candidates at a time and ballot-compact the survivors in candidate
-// order, so each row is written coalesced and in the reference's order.
-__global__ void __launch_bounds__(256) k_build_ref_list(
-    int np, const float4 *__restrict__ ps, const int *__restrict__ sorted,
-    const int *__restrict__ bin_sorted, const int *__restrict__ start,
-    const int *__restrict__ cnum, const int *__restrict__ specbond,
-    const int *__restrict__ num3bond, float box, float ibox, double rv2, int *__restrict__ nlist,
-    int *__restrict__ numneigh, int neigh_alloc, int *__restrict__ status) {
-    const int lane = threadIdx.x & 31;
-    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (s >= np) return;
-    const int i = sorted[s];
-    const float4 pi = ps[s];
-    const int bin = bin_sorted[s];
-    const int n3 = num3bond[i];
-    int bonds[12];
+// Sign bits of dr2 - lim for 8 candidates from place k0 on: bit k of the result is set
+// when candidate k0 + k survives.  IMG: 0 no image, 1 the run's image shift, 2 minimum
+// image per pair.
+template <int IMG>
+__device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 px, float2 py,
+                                              float2 pz, float3 sh, float box, float ibox,
+                                              float2 nlim) {
+    unsigned acc = 0u;
 #pragma unroll
-    for (int l = 0; l < 12; ++l) bonds[l] = specbond[i * 12 + l];
-    int *row = nlist + (size_t)i * (size_t)neigh_alloc;
-    int count = 0;
-    for (int k = 0; k < 27; ++k) {
-        const int c = cnum[bin * 27 + k];
-        const int cs = start[c], ce = start[c + 1];
-        for (int base = cs; base < ce; base += 32) {
-            const int z = base + lane;
-            bool keep = false;
-            int zi = -1;
-            if (z < ce) {
-                const float4 pz = ps[z];
-                zi = sorted[z];
-                float dx = pi.x - pz.x, dy = pi.y - pz.y, dz = pi.z - pz.z;
+    for (int k = 4; k >= 0; k -= 4) {
+        const float4 cx = *reinterpret_cast<const float4 *>(t.x + k0 + k),
+                     cy = *reinterpret_cast<const float4 *>(t.y + k0 + k),
+                     cz = *reinterpret_cast<const float4 *>(t.z + k0 + k);
+#pragma unroll
+        for (int h = 1; h >= 0; --h) {
+            float2 dx = __fadd2_rn(px, h ? make_float2(cx.z, cx.w) : make_float2(cx.x, cx.y)),
+                   dy = __fadd2_rn(py, h ? make_float2(cy.z, cy.w) : make_float2(cy.x, cy.y)),
+                   dz = __fadd2_rn(pz, h ? make_float2(cz.z, cz.w) : make_float2(cz.x, cz.y));
+            if (IMG == 1) {
+                dx = __fadd2_rn(dx, make_float2(sh.x, sh.x));
+                dy = __fadd2_rn(dy, make_float2(sh.y, sh.y));
+                dz = __fadd2_rn(dz, make_float2(sh.z, sh.z));
+            } else if (IMG == 2) {
                 // (b + sign(2^23,b)) - sign(2^23,dx) of :694-697 is rint(b) for |b| < 2^22
-                const float bx = rintf(dx * ibox), by = rintf(dy * ibox), bz = rintf(dz * ibox);
-                dx = dx - bx * box;
-                dy = dy - by * box;
-                dz = dz - bz * box;
-                const float dr2 = dx * dx + dy * dy + dz * dz;
-                keep = (zi != i) && ((double)dr2 < rv2);
-                if (keep) {
-#pragma unroll
-                    for (int l = 0; l < 12; ++l)
-                        if (l < n3 && bonds[l] == zi + 1) keep = false;
-                }
+                dx = make_float2(dx.x - rintf(dx.x * ibox) * box, dx.y - rintf(dx.y * ibox) * box);
+                dy = make_float2(dy.x - rintf(dy.x * ibox) * box, dy.y - rintf(dy.y * ibox) * box);
+                dz = make_float2(dz.x - rintf(dz.x * ibox) * box, dz.y - rintf(dz.y * ibox) * box);
             }
-            const unsigned m = __ballot_sync(FULL, keep);
-            if (keep) {
-                const int at = count + __popc(m & ((1u << lane) - 1u));
-                if (at < neigh_alloc) row[at] = zi + 1;
+            const float2 r2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)),
+                                         __fmul2_rn(dz, dz));
+            float2 d = __fadd2_rn(r2, nlim);
+            if (IMG == 2) {  // a coordinate that is not finite survives nowhere
+                d.x = r2.x < -nlim.x ? -1.0f : 1.0f;
+                d.y = r2.y < -nlim.y ? -1.0f : 1.0f;
             }
-            count += __popc(m);
+            acc = __funnelshift_l(__float_as_uint(d.y), acc, 1);
+            acc = __funnelshift_l(__float_as_uint(d.x), acc, 1);
         }
     }
-    if (lane == 0) {
-        numneigh[i] = count;
-        atomicMax(&status[sofia::ST_MAXCOUNT], count);
+    return acc;
+}
+
+__global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
+    int np, int ncell, int D, const float4 *__restrict__ pair, const int *__restrict__ slot_of,
+    const int *__restrict__ start, const int *__restrict__ chunk,
+    const int *__restrict__ specbond, const int *__restrict__ num3bond, float box, float ibox,
+    float lim, int *__restrict__ nlist, int *__restrict__ numneigh, int neigh_alloc,
+    int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
+    __shared__ __align__(16) ListTile s_tile[LIST_WARPS];
+    __shared__ int s_seg[LIST_WARPS][3][27];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int job = blockIdx.x * LIST_WARPS + w;
+    if (job >= chunk[ncell] || status[sofia::ST_CELLOVER]) return;  // an unsorted cell fails the call
+    const bool shift = D >= 5 && !status[sofia::ST_UNWRAPPED];
+    // the chunk's cell: the last one whose first chunk is not past this one
+    int bin = 0;
+    for (int lo = 0, hi = ncell - 1; lo <= hi;) {
+        const int mid = (lo + hi) >> 1;
+        if (chunk[mid] <= job) {
+            bin = mid;
+            lo = mid + 1;
+        } else {
+            hi = mid - 1;
+        }
     }
+    // stencil cell `lane` in the reference's order: 13 first, then 0..26 without it
+    int c = 0, st = 0, en = 0, code = 0;
+    if (lane < 27) {
+        const int k = lane == 0 ? 13 : (lane <= 13 ? lane - 1 : lane);
+        const int icz = bin / (D * D);
+        const int icy = (bin - icz * D * D) / D;
+        const int icx = bin - icy * D - icz * D * D;
+        const int zc = icz + k / 9 - 1, yc = icy + (k / 3) % 3 - 1, xc = icx + k % 3 - 1;
+        // sign of rint(dx * ibox) across the wrap: -1 from the low side to the high end
+        const int wx = xc < 0 ? -1 : (xc >= D ? 1 : 0), wy = yc < 0 ? -1 : (yc >= D ? 1 : 0),
+                  wz = zc < 0 ? -1 : (zc >= D ? 1 : 0);
+        c = (xc - wx * D) + (yc - wy * D) * D + (zc - wz * D) * D * D;
+        code = (wx + 1) | ((wy + 1) << 2) | ((wz + 1) << 4);
+        st = start[c];
+        en = start[c + 1];
+    }
+    // runs of cells that are adjacent in memory and share the image
+    const int pc = __shfl_up_sync(FULL, c, 1), pcode = __shfl_up_sync(FULL, code, 1);
+    const bool head = lane < 27 && (lane == 0 || c != pc + 1 || (shift && code != pcode));
+    const unsigned heads = __ballot_sync(FULL, head);
+    const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+    const int tail = later ? lane + __ffs(later) - 1 : 26;
+    en = __shfl_sync(FULL, en, tail);
+    if (head) {
+        const int at = __popc(heads & ((1u << lane) - 1u));
+        s_seg[w][0][at] = st;
+        s_seg[w][1][at] = en;
+        s_seg[w][2][at] = code;
+    }
+    const int nseg = __popc(heads);
+    // atom a of the chunk; its lanes share the places of the atom (q = 3, last mark) and
+    // of its up to 12 partners (partner 4l + q is mark l of lane q)
+    const int a = lane & 7, q = lane >> 3;
+    const int s = start[bin] + LIST_ATOMS * (job - chunk[bin]) + a;
+    const bool live = s < start[bin + 1];
+    float2 px = make_float2(0.0f, 0.0f), py = px, pz = px;
+    int id = 0, mark[4] = {-1, -1, -1, -1}, first = INT_MAX, last = -1;
+    if (live) {
+        const float4 p = pair[s];
+        px = make_float2(-p.x, -p.x);
+        py = make_float2(-p.y, -p.y);
+        pz = make_float2(-p.z, -p.z);
+        id = __float_as_int(p.w);
+        const int n3 = min(num3bond[id], 12);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            if (4 * l + q >= n3) continue;
+            const int b = specbond[id * 12 + 4 * l + q];
+            if (b >= 1 && b <= np) mark[l] = slot_of[b - 1];  // others exclude nothing
+        }
+        if (q == 3) mark[3] = s;
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            if (mark[l] >= 0) {
+                first = min(first, mark[l]);
+                last = max(last, mark[l]);
+            }
+    }
+    const int mfirst = __reduce_min_sync(FULL, first), mlast = __reduce_max_sync(FULL, last);
+    const float mylim = live ? -lim : 1.0f;  // without an atom nothing survives (dr2 < -1)
+    const float2 nlim = make_float2(mylim, mylim);
+    const unsigned below = (1u << lane) - 1u, bit = 1u << lane;
+    int *row[LIST_ATOMS];
+    int count[LIST_ATOMS];
+#pragma unroll
+    for (int k = 0; k < LIST_ATOMS; ++k) {
+        row[k] = nlist + (size_t)__shfl_sync(FULL, id, k) * (size_t)neigh_alloc;
+        count[k] = 0;
+    }
+    ListTile &tile = s_tile[w];
+    __syncwarp();
+    for (int g = 0; g < nseg; ++g) {
+        const int b0 = s_seg[w][0][g], b1 = s_seg[w][1][g], cd = s_seg[w][2][g];
+        const float3 sh = make_float3((float)(1 - (cd & 3)) * box,
+                                      (float)(1 - ((cd >> 2) & 3)) * box,
+                                      (float)(1 - ((cd >> 4) & 3)) * box);
+        // a place past the run is infinitely far
+        const float far = __int_as_float(0x7f800000);
+        float4 next = make_float4(far, far, far, 0.0f);
+        if (b0 + lane < b1) next = pair[b0 + lane];
+        for (int base = b0; base < b1; base += 32) {
+            const float4 p = next;
+            next = make_float4(far, far, far, 0.0f);
+            if (base + 32 + lane < b1) next = pair[base + 32 + lane];
+            __syncwarp();
+            tile.x[lane] = p.x;
+            tile.y[lane] = p.y;
+            tile.z[lane] = p.z;
+            __syncwarp();
+#define SOFIA_TILE_ARGS tile, 8 * q, px, py, pz, sh, box, ibox, nlim
+            unsigned m = !shift ? list_tile<2>(SOFIA_TILE_ARGS)
+                       : cd != 21 ? list_tile<1>(SOFIA_TILE_ARGS) : list_tile<0>(SOFIA_TILE_ARGS);
+#undef SOFIA_TILE_ARGS
+            m <<= 8 * q;
+            m |= __shfl_xor_sync(FULL, m, 8);
+            m |= __shfl_xor_sync(FULL, m, 16);
+            if (base <= mlast && base + 32 > mfirst) {
+                unsigned skip = 0u;
+#pragma unroll
+                for (int l = 0; l < 4; ++l) {
+                    const unsigned d = (unsigned)(mark[l] - base);
+                    if (d < 32u) skip |= 1u << d;
+                }
+                skip |= __shfl_xor_sync(FULL, skip, 8);
+                skip |= __shfl_xor_sync(FULL, skip, 16);
+                m &= ~skip;
+            }
+            const int cand = __float_as_int(p.w) + 1;
+#pragma unroll
+            for (int k = 0; k < LIST_ATOMS; ++k) {
+                const unsigned mk = __shfl_sync(FULL, m, k);
+                const int at = count[k] + __popc(mk & below);
+                if ((mk & bit) && at < neigh_alloc) row[k][at] = cand;
+                count[k] += __popc(mk);
+            }
+        }
+    }
+    int most = 0;
+#pragma unroll
+    for (int k = 0; k < LIST_ATOMS; ++k) {
+        if (lane == k && live) numneigh[id] = count[k];
+        most = max(most, count[k]);
+    }
+    if (lane == 0) atomicMax(&status[sofia::ST_MAXCOUNT], most);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -673,9 +869,11 @@ int check_status(sofia_nb_ctx *ctx) {
     return SOFIA_OK;
 }
 
-// Bin + sort + stencil shared by sofia_cell_sort and sofia_neighbor_build.
+// Bin + sort shared by sofia_cell_sort and sofia_neighbor_build.  list: the sorted
+// positions go to pos_pair in the list build's form, with slot_of, instead of to
+// pos_sorted.
 int cell_prepare(sofia_nb_ctx *ctx, int np, const float4 *dpos, float box, float cut_coul,
-                 float rcut, int descending, int *ncellT_out, int *ncellD_out) {
+                 float rcut, int descending, bool list, int *ncellT_out, int *ncellD_out) {
     float rn;
     int nt, nd;
     sofia::cell_grid(box, cut_coul, rcut, &rn, &nt, &nd);
@@ -683,30 +881,30 @@ int cell_prepare(sofia_nb_ctx *ctx, int np, const float4 *dpos, float box, float
         return sofia::fail(ctx, SOFIA_EINVAL, "invalid cell grid (ncellD^3 != ncellT)%s");
     SOFIA_CUDA(ctx, ctx->cell_of.ensure(sizeof(int) * (size_t)np));
     SOFIA_CUDA(ctx, ctx->cell_count.ensure(sizeof(int) * (size_t)(nt + 1)));
-    SOFIA_CUDA(ctx, ctx->cell_fill.ensure(sizeof(int) * (size_t)(nt + 1)));
-    SOFIA_CUDA(ctx, ctx->cell_start.ensure(sizeof(int) * (size_t)(nt + 1)));
+    SOFIA_CUDA(ctx, ctx->cell_rank.ensure(sizeof(int) * (size_t)np));
+    SOFIA_CUDA(ctx, ctx->cell_start.ensure(sizeof(int) * 2 * (size_t)(nt + 1)));
     SOFIA_CUDA(ctx, ctx->sorted_idx.ensure(sizeof(int) * (size_t)np * 2));
-    SOFIA_CUDA(ctx, ctx->pos_sorted.ensure(sizeof(float4) * (size_t)np));
-    SOFIA_CUDA(ctx, ctx->cnum.ensure(sizeof(int) * 27 * (size_t)nt));
+    if (list) {
+        SOFIA_CUDA(ctx, ctx->pos_pair.ensure(sizeof(float4) * (size_t)np));
+        SOFIA_CUDA(ctx, ctx->slot_of.ensure(sizeof(int) * (size_t)np));
+    } else {
+        SOFIA_CUDA(ctx, ctx->pos_sorted.ensure(sizeof(float4) * (size_t)np));
+    }
     cudaStream_t st = ctx->stream;
-    SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t) * sofia::ST_NSLOTS, st));
-    SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->cell_count.p, 0, sizeof(int) * (size_t)(nt + 1), st));
-    SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->cell_fill.p, 0, sizeof(int) * (size_t)(nt + 1), st));
     const double irn = 1.0 / (double)rn;
-    k_bin_atoms<<<sofia::grid_for(np, 256), 256, 0, st>>>(np, dpos, (double)box, irn, nd,
-                                                          ctx->cell_of.as<int>(),
-                                                          ctx->cell_count.as<int>(), ctx->d_status);
-    k_scan_block<<<1, 1024, 0, st>>>(nt, ctx->cell_count.as<int>(), ctx->cell_start.as<int>());
-    int *sorted = ctx->sorted_idx.as<int>();
-    k_scatter<<<sofia::grid_for(np, 256), 256, 0, st>>>(np, ctx->cell_of.as<int>(),
-                                                        ctx->cell_start.as<int>(),
-                                                        ctx->cell_fill.as<int>(), sorted);
-    k_sort_cells<<<nt, 256, 0, st>>>(nt, ctx->cell_start.as<int>(), sorted, descending,
-                                     ctx->d_status);
-    int *bin_sorted = sorted + np;
-    k_gather_sorted<<<sofia::grid_for(np, 256), 256, 0, st>>>(
-        np, sorted, dpos, ctx->cell_of.as<int>(), ctx->pos_sorted.as<float4>(), bin_sorted);
-    k_stencil<<<sofia::grid_for(nt, 128), 128, 0, st>>>(nt, nd, ctx->cnum.as<int>());
+    int *sorted = ctx->sorted_idx.as<int>(), *bin_sorted = sorted + np;
+    int *count = ctx->cell_count.as<int>(), *start = ctx->cell_start.as<int>(),
+        *rank = ctx->cell_rank.as<int>(), *cell_of = ctx->cell_of.as<int>();
+    sofia::launch_pdl(k_clear_cells, sofia::grid_for(nt + 1, 256), 256, 0, st, nt + 1, count,
+                      ctx->d_status);
+    sofia::launch_pdl(k_bin_atoms, sofia::grid_for(np, 256), 256, 0, st, np, dpos, (double)box,
+                      irn, nd, cell_of, rank, count, ctx->d_status);
+    sofia::launch_pdl(k_scan_block, 1, 1024, 0, st, nt, count, start, start + nt + 1);
+    sofia::launch_pdl(k_scatter, sofia::grid_for(np, 256), 256, 0, st, np, cell_of, start, rank,
+                      sorted);
+    sofia::launch_pdl(k_sort_cells, nt, 256, 0, st, nt, start, sorted, descending, dpos,
+                      ctx->pos_sorted.as<float4>(), list ? ctx->pos_pair.as<float4>() : nullptr,
+                      ctx->slot_of.as<int>(), bin_sorted, ctx->d_status);
     SOFIA_CUDA(ctx, cudaGetLastError());
     *ncellT_out = nt;
     *ncellD_out = nd;
@@ -743,7 +941,7 @@ extern "C" int sofia_cell_sort(sofia_nb_ctx *ctx, int np, const sofia_ainfo *pos
     int rc = sofia::stage_in(ctx, position, sizeof(float4) * (size_t)np, 0, &dpos);
     if (rc) return rc;
     int nt, nd;
-    rc = cell_prepare(ctx, np, (const float4 *)dpos, box, cut_coul, rcut, 1, &nt, &nd);
+    rc = cell_prepare(ctx, np, (const float4 *)dpos, box, cut_coul, rcut, 1, false, &nt, &nd);
     if (rc) return rc;
     sofia::OutArg o_tt, o_ttb, o_st, o_en, o_ab, o_ps;
     if ((rc = sofia::stage_out(ctx, tt, sizeof(int) * (size_t)np, 1, &o_tt))) return rc;
@@ -788,7 +986,7 @@ extern "C" int sofia_neighbor_build(sofia_nb_ctx *ctx, int np, const sofia_ainfo
     if ((rc = sofia::stage_in(ctx, specbond, sizeof(int) * 12 * (size_t)np, 1, &dsb))) return rc;
     if ((rc = sofia::stage_in(ctx, num3bond, sizeof(int) * (size_t)np, 2, &dn3))) return rc;
     int nt, nd;
-    if ((rc = cell_prepare(ctx, np, (const float4 *)dpos, box, cut_coul, rcut, 0, &nt, &nd)))
+    if ((rc = cell_prepare(ctx, np, (const float4 *)dpos, box, cut_coul, rcut, 0, true, &nt, &nd)))
         return rc;
     // the list lands in the caller's device buffer, or in the resident buffer
     int32_t *dlist;
@@ -806,12 +1004,16 @@ extern "C" int sofia_neighbor_build(sofia_nb_ctx *ctx, int np, const sofia_ainfo
         SOFIA_CUDA(ctx, ctx->res_numneigh.ensure(sizeof(int) * (size_t)np));
         dnum = ctx->res_numneigh.as<int32_t>();
     }
-    const int *sorted = ctx->sorted_idx.as<int>();
-    const long threads = (long)np * 32;
-    k_build_ref_list<<<sofia::grid_for(threads, 256), 256, 0, st>>>(
-        np, ctx->pos_sorted.as<float4>(), sorted, sorted + np, ctx->cell_start.as<int>(),
-        ctx->cnum.as<int>(), (const int *)dsb, (const int *)dn3, box,
-        (float)(1.0 / (double)box), rv2, dlist, dnum, neigh_alloc, ctx->d_status);
+    // the smallest float that is not below rv2: dr2 < lim decides as (double)dr2 < rv2
+    float lim = (float)rv2;
+    if ((double)lim < rv2) lim = nextafterf(lim, INFINITY);
+    const int *start = ctx->cell_start.as<int>();
+    // at most one partial chunk per cell
+    sofia::launch_pdl(k_build_ref_list, sofia::grid_for((long)np / LIST_ATOMS + nt, LIST_WARPS),
+                      32 * LIST_WARPS, 0, st, np, nt, nd, ctx->pos_pair.as<float4>(),
+                      ctx->slot_of.as<int>(), start, start + nt + 1, (const int *)dsb,
+                      (const int *)dn3, box, (float)(1.0 / (double)box), lim, dlist, dnum,
+                      neigh_alloc, ctx->d_status);
     SOFIA_CUDA(ctx, cudaGetLastError());
     if ((rc = check_status(ctx))) return rc;
     if (ctx->h_status[sofia::ST_CELLOVER])

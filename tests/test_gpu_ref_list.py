@@ -1,0 +1,43 @@
+"""GPU test of the reference-layout list build at the edges of its rules: 2 to 6 cells per
+side (one image per stencil cell is used from 5 on), cells above and below the counting
+sort's size, an odd and an even number of atoms, and coordinates outside the box, which the
+binning takes into the edge cells.  Rows equal the oracle's entry by entry."""
+import numpy as np
+import pytest
+
+from helpers import ref_params
+from molecular_simulation_code_b200 import nonbond as nb
+from molecular_simulation_code_b200.system import make_system
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cut,side", [(17.0, 2), (10.0, 3), (8.5, 4), (7.0, 5), (5.5, 6)])
+@pytest.mark.parametrize("n_wat,outside", [(1400, False), (1401, True)])
+def test_list_rows_exact(ctx, cut, side, n_wat, outside):
+    s = make_system(40, n_wat, 2)
+    p = ref_params(s, cut=cut, pad=1.0)
+    op = O.params(p.alpha, p.box, p.cut_coul, p.rcut, p.neighbor_pad)
+    _, nt, nd = O.cell_grid(op)
+    assert nd == side
+    pos = s.position_aos()
+    if outside:
+        rng = np.random.default_rng(3)
+        hi, lo = rng.permutation(s.np_atoms)[:80].reshape(2, 40)
+        pos[hi, rng.integers(0, 3, 40)] += np.float32(1.3) * s.box
+        pos[lo, rng.integers(0, 3, 40)] = -rng.uniform(0.1, 3.0, 40).astype(np.float32)
+    tt, ttb, st, en, ab = O.bin_sort(op, pos)
+    ps = np.ascontiguousarray(pos[ttb - 1])
+    sb = np.zeros_like(s.specbond)
+    for new in range(s.np_atoms):
+        o = ttb[new] - 1
+        sb[new, :s.num3bond[o]] = tt[s.specbond[o, :s.num3bond[o]] - 1]
+    n3 = np.ascontiguousarray(s.num3bond[ttb - 1])
+    alloc = 9600  # a box of two cells per side lists pairs twice
+    onl, onn, mx = O.build_neighbor_sorted(op, ps, ab, st, en, O.stencil(nt, nd), sb, n3, alloc)
+    assert mx <= alloc
+    nl, nn, na = nb.neighbor_wrapper(ctx, ps, sb, n3, p, neigh_alloc=alloc)
+    assert na == alloc and np.array_equal(nn, onn)
+    used = np.arange(alloc)[None, :] < nn[:, None]
+    assert np.array_equal(nl.reshape(-1, alloc)[used], onl.reshape(-1, alloc)[used])
