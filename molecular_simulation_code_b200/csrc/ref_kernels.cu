@@ -224,7 +224,7 @@ struct ListTile {
 template <int IMG>
 __device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 px, float2 py,
                                               float2 pz, float3 sh, float box, float ibox,
-                                              float2 nlim) {
+                                              float nlim) {
     unsigned acc = 0u;
 #pragma unroll
     for (int k = 4; k >= 0; k -= 4) {
@@ -246,12 +246,15 @@ __device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 
                 dy = make_float2(dy.x - rintf(dy.x * ibox) * box, dy.y - rintf(dy.y * ibox) * box);
                 dz = make_float2(dz.x - rintf(dz.x * ibox) * box, dz.y - rintf(dz.y * ibox) * box);
             }
-            const float2 r2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)),
-                                         __fmul2_rn(dz, dz));
-            float2 d = __fadd2_rn(r2, nlim);
+            // the sums are scalar: packed ones of packed products came out fused, which
+            // moves pairs at exactly the list radius (coordinates on a decimal grid)
+            const float2 xx = __fmul2_rn(dx, dx), yy = __fmul2_rn(dy, dy), zz = __fmul2_rn(dz, dz);
+            const float r0 = __fadd_rn(__fadd_rn(xx.x, yy.x), zz.x),
+                        r1 = __fadd_rn(__fadd_rn(xx.y, yy.y), zz.y);
+            float2 d = make_float2(__fadd_rn(r0, nlim), __fadd_rn(r1, nlim));
             if (IMG == 2) {  // a coordinate that is not finite survives nowhere
-                d.x = r2.x < -nlim.x ? -1.0f : 1.0f;
-                d.y = r2.y < -nlim.y ? -1.0f : 1.0f;
+                d.x = r0 < -nlim ? -1.0f : 1.0f;
+                d.y = r1 < -nlim ? -1.0f : 1.0f;
             }
             acc = __funnelshift_l(__float_as_uint(d.y), acc, 1);
             acc = __funnelshift_l(__float_as_uint(d.x), acc, 1);
@@ -343,8 +346,7 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
             }
     }
     const int mfirst = __reduce_min_sync(FULL, first), mlast = __reduce_max_sync(FULL, last);
-    const float mylim = live ? -lim : 1.0f;  // without an atom nothing survives (dr2 < -1)
-    const float2 nlim = make_float2(mylim, mylim);
+    const float nlim = live ? -lim : 1.0f;  // without an atom nothing survives (dr2 < -1)
     const unsigned below = (1u << lane) - 1u, bit = 1u << lane;
     int *row[LIST_ATOMS];
     int count[LIST_ATOMS];

@@ -1,7 +1,8 @@
 """GPU test of the reference-layout list build at the edges of its rules: 2 to 6 cells per
 side (one image per stencil cell is used from 5 on), cells above and below the counting
-sort's size, an odd and an even number of atoms, and coordinates outside the box, which the
-binning takes into the edge cells.  Rows equal the oracle's entry by entry."""
+sort's size, an odd and an even number of atoms, coordinates outside the box, which the
+binning takes into the edge cells, and coordinates on a grid of 0.01 A, where many pairs lie
+at exactly the list radius and every product has to round by itself.  Rows equal the oracle's entry by entry."""
 import numpy as np
 import pytest
 
@@ -14,14 +15,18 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("cut,side", [(17.0, 2), (10.0, 3), (8.5, 4), (7.0, 5), (5.5, 6)])
-@pytest.mark.parametrize("n_wat,outside", [(1400, False), (1401, True)])
-def test_list_rows_exact(ctx, cut, side, n_wat, outside):
+@pytest.mark.parametrize("n_wat,outside,grid", [(1400, False, False), (1401, True, False),
+                                                (1400, False, True)])
+def test_list_rows_exact(ctx, cut, side, n_wat, outside, grid):
     s = make_system(40, n_wat, 2)
     p = ref_params(s, cut=cut, pad=1.0)
     op = O.params(p.alpha, p.box, p.cut_coul, p.rcut, p.neighbor_pad)
     _, nt, nd = O.cell_grid(op)
     assert nd == side
     pos = s.position_aos()
+    if grid:
+        pos[:, :3] = np.round(pos[:, :3], 2)
+        pos[:, :3] = np.minimum(pos[:, :3], s.box)
     if outside:
         rng = np.random.default_rng(3)
         hi, lo = rng.permutation(s.np_atoms)[:80].reshape(2, 40)
