@@ -452,16 +452,76 @@ __host__ DsfConst make_const(float box, float ibox, double rcut2, double cut_cou
     return c;
 }
 
-// lj_cut_coul_dsf_nonewton_NOMIC, mod_force_nonbond.f90:105-196.  One warp per
-// atom i; lane l takes neighbours l, l+32, ... of the row (coalesced index
-// loads), keeps FP64 partial sums and the warp combines them with a fixed
-// butterfly, so results are bit-reproducible run to run.
+// Row sweep of the two reference-layout force kernels: one warp per atom i looks at
+// its row's neighbours, queues those that can be inside a cut-off in shared memory, and
+// calls pair(neighbour) with a full warp of them: the list reaches to cut-off + skin,
+// so at 10 + 2 A 42 % of a row contributes nothing.  near(neighbour's record) must be
+// true for every pair that contributes.  The rows come from memory and every
+// neighbour's record waits for its index, so 4 x 32 indices are read at a time, one
+// round ahead, and their records together.  Every lane's pairs stay in row order, so
+// sums are reproducible run to run.
+constexpr int SWEEP = 4;
+constexpr int SWEEP_QUEUE = 32 * (SWEEP + 1);
+template <class Near, class Pair>
+__device__ __forceinline__ void sweep_row(int np, int ntypes, const float4 *__restrict__ pos,
+                                          const int *__restrict__ row, int num, int *queue,
+                                          Near near, Pair pair) {
+    const int lane = threadIdx.x & 31;
+    int next[SWEEP];
+#pragma unroll
+    for (int u = 0; u < SWEEP; ++u) next[u] = 32 * u + lane < num ? row[32 * u + lane] : 0;
+    int held = 0;
+    for (int base = 0; base < num; base += 32 * SWEEP) {
+        int neigh[SWEEP];
+        float4 pj[SWEEP];
+#pragma unroll
+        for (int u = 0; u < SWEEP; ++u) {
+            neigh[u] = next[u] - 1;
+            const bool ok = (unsigned)neigh[u] < (unsigned)np;
+            // a record that is not there has no type
+            pj[u] = ok ? pos[neigh[u]] : make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
+            const int j = base + 32 * (SWEEP + u) + lane;
+            next[u] = j < num ? row[j] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < SWEEP; ++u) {
+            const bool keep = (unsigned)(__float_as_int(pj[u].w) - 1) < (unsigned)ntypes &&
+                              near(pj[u]);
+            const unsigned m = __ballot_sync(FULL, keep);
+            if (keep) queue[held + __popc(m & ((1u << lane) - 1u))] = neigh[u];
+            held += __popc(m);
+        }
+        __syncwarp();
+        const bool last = base + 32 * SWEEP >= num;
+        int head = 0;
+        while (held >= 32 || (last && held > 0)) {
+            if (lane < held) pair(queue[head + lane]);
+            head += 32;
+            held -= 32;
+        }
+        if (held > 0) {  // the rest moves to the front (less than a warp of it)
+            const int rest = lane < held ? queue[head + lane] : 0;
+            __syncwarp();
+            if (lane < held) queue[lane] = rest;
+        }
+        __syncwarp();
+    }
+}
+
+// lj_cut_coul_dsf_nonewton_NOMIC, mod_force_nonbond.f90:105-196, FP64 over the row of
+// atom i (sweep_row); the warp combines the lanes' partial sums with a fixed butterfly.
+// A real*4 distance with a bound on its rounding screens the row; pairs inside are
+// evaluated in FP64 throughout, with one reciprocal square root for r, 1/r and 1/r^2.
+// 45,255 atoms: 269 us (FP64 and conversion pipes at 40 %); 415 us with every listed
+// pair evaluated and a square root and three divisions each, 399 us with the screen
+// but one index and one record in flight per lane.
 __global__ void __launch_bounds__(256) k_force_ref(
     int np, const float4 *__restrict__ pos, const float *__restrict__ q,
     const float *__restrict__ lj1, const float *__restrict__ lj2, const float *__restrict__ lj3,
     const float *__restrict__ lj4, int ntypes, const int *__restrict__ nlist,
     const int *__restrict__ numneigh, int neigh_alloc, DsfConst k, float *__restrict__ ff,
     double *__restrict__ pe) {
+    __shared__ int s_queue[8][SWEEP_QUEUE];
     const int lane = threadIdx.x & 31;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= np) return;
@@ -470,34 +530,45 @@ __global__ void __launch_bounds__(256) k_force_ref(
     const int itype = __float_as_int(pi.w);
     const double qtmp = (double)q[i];
     const int ioffset = (itype - 1) * ntypes;
-    const int num = min(numneigh[i], neigh_alloc);
-    const int *row = nlist + (size_t)i * (size_t)neigh_alloc;
     const bool itype_ok = (unsigned)(itype - 1) < (unsigned)ntypes;
+    const int num = itype_ok ? min(numneigh[i], neigh_alloc) : 0;
+    const int *row = nlist + (size_t)i * (size_t)neigh_alloc;
     const double TWO_ALPHA_PI = (2.0 * k.alpha) * k.MY_PIS_INV;
     const double EPA = k.EWALD_P * k.alpha;
     const double AA = k.alpha * k.alpha;
     double ffx = 0.0, ffy = 0.0, ffz = 0.0, pot = 0.0, ec = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
-    for (int j = lane; j < num; j += 32) {
-        const int neigh = row[j] - 1;
-        if ((unsigned)neigh >= (unsigned)np) continue;
+    // Screen: each component of the real*4 minimum-image distance is off by less than
+    // e = 1e-6 |raw difference| summed over the components (the subtraction, the image
+    // product and its subtraction round by 2^-24 of it each), so a pair inside
+    // sqrt(far) has a real*4 square below far + 4 sqrt(far) e + 4 e^2.  A NaN passes.
+    const float far = (float)fmax(k.rcut2, k.cut_coulsq) * 1.00001f, slope = 4.0f * sqrtf(far);
+    auto near = [&](const float4 &pj) {
+        float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const float e = 1e-6f * (fabsf(dx) + fabsf(dy) + fabsf(dz));
+        dx = dx - k.boxf * rintf(dx * k.iboxf);
+        dy = dy - k.boxf * rintf(dy * k.iboxf);
+        dz = dz - k.boxf * rintf(dz * k.iboxf);
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        return !(d2 > far + e * (slope + 4.0f * e));
+    };
+    auto pair = [&](int neigh) {
         const float4 pj = pos[neigh];
         double dx = x1 - (double)pj.x, dy = y1 - (double)pj.y, dz = z1 - (double)pj.z;
         const int jtype = __float_as_int(pj.w);
-        if (!itype_ok || (unsigned)(jtype - 1) >= (unsigned)ntypes) continue;
         // (b + sign(2^52,b)) - sign(2^52,dx) of :144-147 is rint(b) for |b| < 2^51
         const double bx = rint(dx * k.ibox), by = rint(dy * k.ibox), bz = rint(dz * k.ibox);
         dx = dx - k.box * bx;
         dy = dy - k.box * by;
         dz = dz - k.box * bz;
         const double dr2 = dx * dx + dy * dy + dz * dz;
-        const double dr2i = 1.0 / dr2;
+        const double dri = rsqrt(dr2);
+        const double dr2i = dri * dri;
+        const double r = dr2 == 0.0 ? 0.0 : dr2 * dri;  // 0, not 0 * inf, for coincident atoms
         double dr6i = dr2i * dr2i * dr2i;
         if (dr2 > k.rcut2) dr6i = 0.0;
         const int off = ioffset + jtype - 1;
         const double forcelj = dr6i * ((double)lj1[off] * dr6i - (double)lj2[off]);
         pot = pot + dr6i * (dr6i * (double)lj3[off] - (double)lj4[off]);
-        const double r = sqrt(dr2);
-        const double dri = 1.0 / r;
         double prefactor = k.coulpre * qtmp * (double)q[neigh] * dri;
         if (dr2 > k.cut_coulsq) prefactor = 0.0;
         const double erfcd = exp(-((AA * r) * r));
@@ -513,7 +584,8 @@ __global__ void __launch_bounds__(256) k_force_ref(
         vx = vx + dx * dx * force;
         vy = vy + dy * dy * force;
         vz = vz + dz * dz * force;
-    }
+    };
+    sweep_row(np, ntypes, pos, row, num, s_queue[threadIdx.x >> 5], near, pair);
     ffx = warp_sum(ffx);
     ffy = warp_sum(ffy);
     ffz = warp_sum(ffz);
@@ -536,20 +608,23 @@ __global__ void __launch_bounds__(256) k_force_ref(
 }
 
 // lj_cut_coul_long_nonewton_NOMIC / _MIC (mod_force_nonbond.f90:300-400, :201-298):
-// the real-space Ewald term of the PME path.  Same warp-per-atom layout as
+// the real-space Ewald term of the PME path.  Same warp-per-atom sweep as
 // k_force_ref, but every pair quantity is real*4 as in the reference; the
 // mixed-mode statements are promoted to double where Fortran promotes them
 // (dr2i = 1.0d0/dr2, grij = gewald*r, t, the erfc polynomial, forcecoul) and
 // force/virial products are added into double sums.  This unit is compiled
 // without FMA contraction, so each float operation rounds as written.  The
 // real*4 exp is the correctly rounded single-precision value obtained by
-// rounding the double-precision exp.
+// rounding the double-precision exp.  dr2i is the real*4 division: rounding the
+// double quotient of two real*4 values to real*4 gives the same bits (53 >= 2*24 + 2).
+// The sweep's screen is the reference's own real*4 distance, so it is exact.
 __global__ void __launch_bounds__(256) k_force_long_ref(
     int np, const float4 *__restrict__ pos, const float *__restrict__ q,
     const float *__restrict__ lj1, const float *__restrict__ lj2, const float *__restrict__ lj3,
     const float *__restrict__ lj4, int ntypes, const int *__restrict__ nlist,
     const int *__restrict__ numneigh, int neigh_alloc, DsfConst k, float *__restrict__ ff,
     double *__restrict__ pe) {
+    __shared__ int s_queue[8][SWEEP_QUEUE];
     const int lane = threadIdx.x & 31;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= np) return;
@@ -557,24 +632,32 @@ __global__ void __launch_bounds__(256) k_force_long_ref(
     const int itype = __float_as_int(pi.w);
     const float qtmp = q[i];
     const int ioffset = (itype - 1) * ntypes;
-    const int num = min(numneigh[i], neigh_alloc);
-    const int *row = nlist + (size_t)i * (size_t)neigh_alloc;
     const bool itype_ok = (unsigned)(itype - 1) < (unsigned)ntypes;
+    const int num = itype_ok ? min(numneigh[i], neigh_alloc) : 0;
+    const int *row = nlist + (size_t)i * (size_t)neigh_alloc;
     const float box = k.boxf, ibox = k.iboxf, coulpre = k.coulpref;
     double ffx = 0.0, ffy = 0.0, ffz = 0.0, pot = 0.0, ec = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
-    for (int j = lane; j < num; j += 32) {
-        const int neigh = row[j] - 1;
-        if ((unsigned)neigh >= (unsigned)np) continue;
-        const float4 pj = pos[neigh];
-        const int jtype = __float_as_int(pj.w);
-        if (!itype_ok || (unsigned)(jtype - 1) >= (unsigned)ntypes) continue;
-        float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+    auto image = [&](const float4 &pj, float &dx, float &dy, float &dz) {
+        dx = pi.x - pj.x;
+        dy = pi.y - pj.y;
+        dz = pi.z - pj.z;
         // (b + sign(2^23,b)) - sign(2^23,dx) is rint(b) in real*4 for |b| < 2^22
         dx = dx - box * rintf(dx * ibox);
         dy = dy - box * rintf(dy * ibox);
         dz = dz - box * rintf(dz * ibox);
-        const float dr2 = dx * dx + dy * dy + dz * dz;
-        const float dr2i = (float)(1.0 / (double)dr2);
+        return dx * dx + dy * dy + dz * dz;
+    };
+    const double far = fmax(k.rcut2, k.cut_coulsq);
+    auto near = [&](const float4 &pj) {
+        float dx, dy, dz;
+        return !((double)image(pj, dx, dy, dz) > far);
+    };
+    auto pair = [&](int neigh) {
+        const float4 pj = pos[neigh];
+        const int jtype = __float_as_int(pj.w);
+        float dx, dy, dz;
+        const float dr2 = image(pj, dx, dy, dz);
+        const float dr2i = __fdiv_rn(1.0f, dr2);
         float dr6i = dr2i * dr2i * dr2i;
         if ((double)dr2 > k.rcut2) dr6i = 0.0f;
         const int off = ioffset + jtype - 1;
@@ -598,7 +681,8 @@ __global__ void __launch_bounds__(256) k_force_long_ref(
         vx = vx + (double)(dx * dx * force);
         vy = vy + (double)(dy * dy * force);
         vz = vz + (double)(dz * dz * force);
-    }
+    };
+    sweep_row(np, ntypes, pos, row, num, s_queue[threadIdx.x >> 5], near, pair);
     ffx = warp_sum(ffx);
     ffy = warp_sum(ffy);
     ffz = warp_sum(ffz);
