@@ -282,7 +282,7 @@ __device__ __forceinline__ void pack_body(int bx, int nslots, const int *__restr
                        const double *__restrict__ rz, const double *__restrict__ ix,
                        const double *__restrict__ iy, const double *__restrict__ iz,
                        const float *__restrict__ q, const int *__restrict__ type, double L,
-                       AtomRec *__restrict__ rec, float *__restrict__ recf,
+                       ClusterRec *__restrict__ rec, float *__restrict__ recf,
                        long long *__restrict__ fslot, float4 *__restrict__ bb,
                        const int *__restrict__ cond, double *__restrict__ sref) {
     const int s = bx * blockDim.x + threadIdx.x;
@@ -357,7 +357,9 @@ __device__ __forceinline__ void pack_body(int bx, int nslots, const int *__restr
         r.type = 0;
     }
     if (live) {
-        rec[s] = r;
+        ClusterRec &cr = rec[s / CL];
+        cr.lo[s % CL] = {r.x, r.y};
+        cr.hi[s % CL] = {r.z, r.q, r.type};
         // FP32 copy for the prune, per cluster x[8], y[8], z[8]
         float *rc = recf + (size_t)(s / CL) * (3 * CL) + (s % CL);
         rc[0] = (float)r.x;
@@ -396,7 +398,7 @@ __global__ void k_pack(int nslots, const int *__restrict__ ncl_dev,
                        const double *__restrict__ rz, const double *__restrict__ ix,
                        const double *__restrict__ iy, const double *__restrict__ iz,
                        const float *__restrict__ q, const int *__restrict__ type, double L,
-                       AtomRec *__restrict__ rec, float *__restrict__ recf,
+                       ClusterRec *__restrict__ rec, float *__restrict__ recf,
                        long long *__restrict__ fslot, float4 *__restrict__ bb,
                        const int *__restrict__ cond, double *__restrict__ sref) {
     SOFIA_PDL_ENTRY();
@@ -862,6 +864,12 @@ __device__ __forceinline__ void flush_i(long long *__restrict__ fi, int lane, T 
     fi[5 * 32 + lane] += to_fix<T>(z1);
 }
 
+__device__ __forceinline__ AtomRec load_rec(const ClusterRec *__restrict__ rec, int cl, int at) {
+    const ClusterRec::Lo lo = rec[cl].lo[at];
+    const ClusterRec::Hi hi = rec[cl].hi[at];
+    return AtomRec{lo.x, lo.y, hi.z, hi.q, hi.type};
+}
+
 // Pair kernel on the half cluster-pair list (each atom pair once, Newton's
 // third law).  One warp per i-cluster; lane = jj + 8 q (jj = j atom 0..7,
 // q = 0..3): for every listed j-cluster the lane evaluates the pairs of j atom
@@ -889,7 +897,7 @@ __device__ __forceinline__ void flush_i(long long *__restrict__ fi, int lane, T 
 // batch b adding to slot b % ESLOT in batch order, so they do not either.
 template <typename T, bool EN, bool VIR, bool SAME, bool TRI, int SPLIT>
 __device__ __forceinline__ void pair_body(
-    int bx, int maxcl, const int *__restrict__ ncl_dev, const AtomRec *__restrict__ rec,
+    int bx, int maxcl, const int *__restrict__ ncl_dev, const ClusterRec *__restrict__ rec,
     const int *__restrict__ jlist, const unsigned long long *__restrict__ jmask,
     const int *__restrict__ jcount, int jcap, const float4 *__restrict__ ljtab,
     const PairConst &k, double L, unsigned long long *__restrict__ fslot,
@@ -945,7 +953,7 @@ __device__ __forceinline__ void pair_body(
     const size_t stride = (size_t)maxcl * CL;
     // this lane's share of the reduced j force: component q (3 = none) of j atom jj
     unsigned long long *jdst = fslot + (size_t)(q < 3 ? q : 0) * stride;
-    const AtomRec ri0 = rec[icl * CL + q], ri1 = rec[icl * CL + q + 4];
+    const AtomRec ri0 = load_rec(rec, icl, q), ri1 = load_rec(rec, icl, q + 4);
     const T qiq0 = (T)k.coulpre * (T)ri0.q, qiq1 = (T)k.coulpre * (T)ri1.q;
     const int ti0 = ri0.type * k.ntypes, ti1 = ri1.type * k.ntypes;
     const int t3 = (ri0.type * k.ntypes + ri1.type) * k.ntypes;  // this lane's TRI row
@@ -973,7 +981,7 @@ __device__ __forceinline__ void pair_body(
                 const unsigned long long mm = __shfl_sync(FULL, mym, e);
                 const int jc = w & ((1 << IMG_SHIFT) - 1);
                 const int img = w >> IMG_SHIFT;
-                const AtomRec rj = rec[jc * CL + jj];
+                const AtomRec rj = load_rec(rec, jc, jj);
                 // j position in the image the entry pairs with
                 const double xj = rj.x + s_sh[img * 3 + 0];
                 const double yj = rj.y + s_sh[img * 3 + 1];
@@ -1193,7 +1201,7 @@ __device__ __forceinline__ void pair_body(
 }
 template <typename T, bool EN, bool VIR, bool SAME, bool TRI = false, int SPLIT = 1>
 __global__ void __launch_bounds__((pair_block<T, EN>()), (pair_minb<T, EN>())) k_pair(
-    int maxcl, const int *__restrict__ ncl_dev, const AtomRec *__restrict__ rec,
+    int maxcl, const int *__restrict__ ncl_dev, const ClusterRec *__restrict__ rec,
     const int *__restrict__ jlist, const unsigned long long *__restrict__ jmask,
     const int *__restrict__ jcount, int jcap, const float4 *__restrict__ ljtab, PairConst k,
     unsigned long long *__restrict__ fslot, double *__restrict__ energy) {
@@ -1542,7 +1550,7 @@ static int sys_alloc(Sys *s) {
     SOFIA_CUDA(ctx, s->col_key.ensure(sizeof(float) * n));
     const size_t maxcl = (size_t)s->max_clusters;
     SOFIA_CUDA(ctx, s->slot_orig.ensure(sizeof(int) * maxcl * CL + sizeof(int) * maxcl));
-    SOFIA_CUDA(ctx, s->rec.ensure(sizeof(AtomRec) * maxcl * CL));
+    SOFIA_CUDA(ctx, s->rec.ensure(sizeof(ClusterRec) * maxcl));
     SOFIA_CUDA(ctx, s->sref.ensure((6 * sizeof(double) + sizeof(float) + sizeof(int)) * maxcl * CL));
     SOFIA_CUDA(ctx, s->recf.ensure(sizeof(float) * 3 * maxcl * CL));
     SOFIA_CUDA(ctx, s->fslot.ensure(sizeof(long long) * 3 * maxcl * CL));
@@ -1617,7 +1625,7 @@ static void sys_pack(Sys *s, const int *cond) {
         s->x[1].as<double>(), s->x[2].as<double>(), s->xref[0].as<double>(),
         s->xref[1].as<double>(), s->xref[2].as<double>(), s->img[0].as<double>(),
         s->img[1].as<double>(), s->img[2].as<double>(), s->q.as<float>(), s->type.as<int>(), s->L,
-        s->rec.as<AtomRec>(), s->recf.as<float>(), s->fslot.as<long long>(), s->bb.as<float4>(),
+        s->rec.as<ClusterRec>(), s->recf.as<float>(), s->fslot.as<long long>(), s->bb.as<float4>(),
         cond, s->sref.as<double>());
     s->launches += 1;
 }
@@ -1872,7 +1880,7 @@ static void launch_pair_one(Sys *s, const PairConst &k) {
     launch_pdl(k_pair<T, EN, VIR, true, TRI, SPLIT>,
                grid_for((long)s->max_clusters * SPLIT * 32, block), block,
                pair_smem(s->ntypes, TRI, EN), s->ctx->stream, s->max_clusters,
-               s->nclusters.as<int>(), s->rec.as<AtomRec>(), s->ilist.as<int>(),
+               s->nclusters.as<int>(), s->rec.as<ClusterRec>(), s->ilist.as<int>(),
                s->imask.as<unsigned long long>(), s->icount.as<int>(), s->jcap,
                s->ljtab.as<float4>(), k, s->fslot.as<unsigned long long>(),
                s->energy.as<double>());
@@ -2733,7 +2741,7 @@ void repdev_fill_pair(const Sys *s, RepDev *d) {
     d->cl_col = s->slot_orig.as<int>() + (size_t)s->max_clusters * CL;
     d->atom_slot = s->atom_slot.as<int>();
     d->col_key = s->col_key.as<float>();
-    d->rec = s->rec.as<AtomRec>();
+    d->rec = s->rec.as<ClusterRec>();
     d->sref = s->sref.as<double>();
     d->recf = s->recf.as<float>();
     d->bb = s->bb.as<float4>();

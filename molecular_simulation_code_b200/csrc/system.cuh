@@ -4,9 +4,9 @@
 //   global-order atom state   x/v (double SoA), f (int64 fixed point SoA),
 //                             type (int32), q (float), inverse mass (double),
 //                             positions at the last list build (double SoA)
-//   cluster order             AtomRec[slot] = {double x,y,z; float q; int type}
-//                             (32 B, two 16 B loads), slot -> global index,
-//                             8 slots per cluster, clusters grouped by xy column
+//   cluster order             ClusterRec[cluster] = {double x,y}[8], {double z;
+//                             float q; int type}[8] (256 B, two 16 B loads per
+//                             atom), slot -> global index, 8 slots per cluster, clusters grouped by xy column
 //                             and sorted by z inside a column; an FP32 copy for
 //                             the prune as float x[8], y[8], z[8] per cluster
 //                             (96 B, six 16 B loads)
@@ -29,6 +29,14 @@ struct __align__(16) AtomRec {
     double x, y, z;
     float q;
     int type;
+};
+// The 8 atom records of a cluster as two runs of 16-byte halves: the 8 lanes that
+// load a half from a cluster touch one 128-byte line, where whole 32-byte records
+// in a row would spread each half over two (the pair kernel's record loads are half
+// of its L1 wavefronts that way).
+struct __align__(16) ClusterRec {
+    struct __align__(16) Lo { double x, y; } lo[CL];
+    struct __align__(16) Hi { double z; float q; int type; } hi[CL];
 };
 
 // Device-resident MD state (velocity Verlet + force-form Langevin + SHAKE +
@@ -194,7 +202,7 @@ struct RepDev {
     int *col_count, *col_start, *col_fill, *col_atoms, *col_of, *cl_start, *slot_orig, *cl_col,
         *atom_slot;
     float *col_key;
-    AtomRec *rec;
+    ClusterRec *rec;
     double *sref;
     float *recf;
     float4 *bb;
