@@ -32,6 +32,8 @@ extern "C" int sofia_nb_create(const sofia_nb_params *params, sofia_nb_ctx **out
         sofia_nb_destroy(ctx);
         return SOFIA_ECUDA;
     }
+    sofia::transfer_open();
+    ctx->opened = true;
     *out = ctx;
     return SOFIA_OK;
 }
@@ -58,7 +60,10 @@ extern "C" int sofia_nb_destroy(sofia_nb_ctx *ctx) {
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->h_red) cudaFreeHost(ctx->h_red);
+    for (auto &x : ctx->xstream)
+        if (x) cudaStreamDestroy(x);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->opened) sofia::transfer_close();
     delete ctx;
     return SOFIA_OK;
 }

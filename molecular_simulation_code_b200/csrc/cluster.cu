@@ -361,6 +361,7 @@ extern "C" int sofia_greatest_cluster(sofia_nb_ctx *ctx, int np, const sofia_ain
         return SOFIA_OK;
     }
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dpos, *dgid;
@@ -430,17 +431,15 @@ extern "C" int sofia_greatest_cluster(sofia_nb_ctx *ctx, int np, const sofia_ain
     // size, cluster number and density-list overflows into pinned words
     int32_t *res = ctx->h_status;
     SOFIA_CUDA(ctx, cudaMemcpyAsync(res, a.result, sizeof(int32_t) * 3, cudaMemcpyDeviceToHost, st));
-    if (denstrack)
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(denstrack, a.denstrack, sizeof(int) * n,
-                                        sofia::is_device_ptr(denstrack) ? cudaMemcpyDeviceToDevice
-                                                                        : cudaMemcpyDeviceToHost,
-                                        st));
-    if (belongsto)
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(belongsto, a.label, sizeof(int) * n,
-                                        sofia::is_device_ptr(belongsto) ? cudaMemcpyDeviceToDevice
-                                                                        : cudaMemcpyDeviceToHost,
-                                        st));
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
+    for (const auto &o : {std::make_pair(denstrack, a.denstrack), std::make_pair(belongsto, a.label)}) {
+        if (!o.first) continue;
+        if (sofia::is_device_ptr(o.first))
+            SOFIA_CUDA(ctx, cudaMemcpyAsync(o.first, o.second, sizeof(int) * n,
+                                            cudaMemcpyDeviceToDevice, st));
+        else if ((rc = copies.out(o.first, o.second, sizeof(int) * n)))
+            return rc;
+    }
+    if ((rc = copies.sync())) return rc;
     if (res[2])
         return sofia::fail(ctx, SOFIA_EINVAL, "density list overflow (more than 256 entries)%s");
     *size_out = res[0];

@@ -71,8 +71,17 @@ __host__ __device__ inline uint32_t transpose_8x4(uint32_t x) {
 
 }  // namespace sofia
 
+namespace sofia {
+class HostCopies;
+void transfer_open();   // a context was created
+void transfer_close();  // and destroyed: the last one frees the pinned slots
+}  // namespace sofia
+
 struct sofia_nb_ctx {
     int device = 0;
+    bool opened = false;                                            // counted by transfer_open
+    sofia::HostCopies *copies = nullptr;                            // of the call being served
+    cudaStream_t xstream[4] = {nullptr, nullptr, nullptr, nullptr};  // large host copies
     cudaStream_t stream = nullptr;
     std::string last_error;
     // status words: device array + pinned host mirror
@@ -125,6 +134,37 @@ inline int cuda_fail(sofia_nb_ctx *ctx, cudaError_t e, const char *where,
         if (_e != cudaSuccess) return sofia::cuda_fail((ctx), _e, #call, __FILE__, __LINE__); \
     } while (0)
 
+// The host copies of one call of the C ABI (transfer.cu), made at its start: in()
+// returns with the host array free to reuse, out() may deliver as late as sync(),
+// which also waits for the context's stream.  A call that fails before sync()
+// delivers nothing more.
+class HostCopies {
+  public:
+    explicit HostCopies(sofia_nb_ctx *c);
+    ~HostCopies();
+    HostCopies(const HostCopies &) = delete;
+    HostCopies &operator=(const HostCopies &) = delete;
+    int in(void *dev, const void *host, size_t bytes);
+    int out(void *host, const void *dev, size_t bytes);
+    int sync();
+
+  private:
+    static constexpr int MAX = 16;
+    struct Out {
+        void *host;
+        const char *pinned;
+        size_t bytes;
+    };
+    char *reserve(size_t bytes);
+    sofia_nb_ctx *ctx;
+    HostCopies *outer;  // of a call that this one is part of
+    char *slots[MAX];
+    Out outs[MAX];
+    int nslot = 0, nout = 0;
+    size_t used = 0;
+    bool idle = true;  // no copy of the slots is in flight
+};
+
 // True when p is device (or managed) memory; host pointers are staged.
 inline bool is_device_ptr(const void *p) {
     if (!p) return false;
@@ -137,6 +177,7 @@ inline bool is_device_ptr(const void *p) {
 }
 
 // Returns a device pointer holding `bytes` of input; host data is copied into stage[slot].
+// These three belong to a call that has its HostCopies.
 inline int stage_in(sofia_nb_ctx *ctx, const void *p, size_t bytes, int slot, const void **out) {
     if (!p || bytes == 0) {
         *out = p;
@@ -147,10 +188,8 @@ inline int stage_in(sofia_nb_ctx *ctx, const void *p, size_t bytes, int slot, co
         return SOFIA_OK;
     }
     SOFIA_CUDA(ctx, ctx->stage[slot].ensure(bytes));
-    SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->stage[slot].p, p, bytes, cudaMemcpyHostToDevice,
-                                    ctx->stream));
     *out = ctx->stage[slot].p;
-    return SOFIA_OK;
+    return ctx->copies->in(ctx->stage[slot].p, p, bytes);
 }
 
 // Output helper: returns a device pointer to write to; `host` is set when a copy-back is due.
@@ -173,15 +212,11 @@ inline int stage_out(sofia_nb_ctx *ctx, void *p, size_t bytes, int slot, OutArg 
     SOFIA_CUDA(ctx, ctx->stage[slot].ensure(bytes));
     o->dev = ctx->stage[slot].p;
     o->host = p;
-    if (copy_in_first)
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(o->dev, p, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    return SOFIA_OK;
+    return copy_in_first ? ctx->copies->in(o->dev, p, bytes) : SOFIA_OK;
 }
+// The caller's array is filled by the time of the call's sync().
 inline int finish_out(sofia_nb_ctx *ctx, const OutArg &o) {
-    if (o.host && o.bytes)
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(o.host, o.dev, o.bytes, cudaMemcpyDeviceToHost,
-                                        ctx->stream));
-    return SOFIA_OK;
+    return o.host && o.bytes ? ctx->copies->out(o.host, o.dev, o.bytes) : SOFIA_OK;
 }
 
 inline int grid_for(long n, int block) { return (int)((n + block - 1) / block); }

@@ -1147,7 +1147,14 @@ extern "C" int sofia_system_md_run(sofia_system *ss, int nsteps, int energy_ever
             }
             ++k;
         }
-        rc = sofia::sys_list_overflow(s);
+        // the status words and the energies come back together
+        int32_t *hs = ctx->h_status;
+        SOFIA_CUDA(ctx, cudaMemcpyAsync(hs, s->status_local.p, sizeof(int32_t) * sofia::ST_NSLOTS,
+                                        cudaMemcpyDeviceToHost, st));
+        SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->h_red, md.ered.p, sizeof(double) * 16,
+                                        cudaMemcpyDeviceToHost, st));
+        SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
+        rc = sofia::sys_list_overflow(s, hs);
         if (rc == SOFIA_ENEEDGROW) {
             // list row capacity grew: restore the segment start and run it again
             sofia::md_drop_graphs(s);
@@ -1160,18 +1167,11 @@ extern "C" int sofia_system_md_run(sofia_system *ss, int nsteps, int energy_ever
             continue;
         }
         if (rc) return rc;
-        int hs[sofia::ST_NSLOTS];
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(hs, s->status_local.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
-        SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
         if (hs[sofia::ST_SHAKE])
             return sofia::fail(ctx, SOFIA_ESTATE, "SHAKE determinant <= 0 (mod_shake.f90:146-153, :267)%s");
         s->shake_nc += hs[sofia::ST_SHAKE_NC];
         md.step += nsteps;
-        if (energies && energy_every > 0) {
-            double e[16];
-            SOFIA_CUDA(ctx, cudaMemcpy(e, md.ered.p, sizeof(double) * 16, cudaMemcpyDeviceToHost));
-            sofia::md_fill_energies(md, e, energies);
-        }
+        if (energies && energy_every > 0) sofia::md_fill_energies(md, ctx->h_red, energies);
         return SOFIA_OK;
     }
     return sofia::fail(ctx, SOFIA_ENEEDGROW, "list capacity kept overflowing%s");
@@ -1226,13 +1226,9 @@ extern "C" int sofia_system_md_forces(sofia_system *ss, int terms, double *f, do
     if (hs[sofia::ST_SHAKE])
         return sofia::fail(ctx, SOFIA_ESTATE, "SHAKE determinant <= 0 (mod_shake.f90:146-153, :267)%s");
     if (f) {
-        const size_t n = (size_t)s->n;
-        std::vector<long long> h(3 * n);
-        for (int d = 0; d < 3; ++d)
-            SOFIA_CUDA(ctx, cudaMemcpy(h.data() + d * n, s->f[d].p, sizeof(long long) * n,
-                                       cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < n; ++i)
-            for (int d = 0; d < 3; ++d) f[3 * i + d] = (double)h[d * n + i] * sofia::FIX_INV;
+        sofia::HostCopies copies(ctx);
+        if ((rc = sofia::forces_out(s, f))) return rc;
+        if ((rc = copies.sync())) return rc;
     }
     if (energies) {
         double e[16];

@@ -1514,6 +1514,28 @@ __global__ void k_aos_to_soa(int n, const float4 *__restrict__ pos, double *__re
     z[i] = (double)p.z;
 }
 
+// The caller's [n][3] state arrays <-> the SoA state.  One thread per value: the
+// AoS side is read or written in order, the SoA side a third of a line at a time.
+__global__ void k_state_in(int n, const double *__restrict__ in, double *__restrict__ x,
+                           double *__restrict__ y, double *__restrict__ z) {
+    SOFIA_PDL_ENTRY();
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 3 * n) return;
+    const int i = e / 3, d = e - 3 * i;
+    (d == 0 ? x : d == 1 ? y : z)[i] = in[e];
+}
+__device__ __forceinline__ double state_value(double v) { return v; }
+__device__ __forceinline__ double state_value(long long v) { return (double)v * FIX_INV; }
+template <typename T>
+__global__ void k_state_out(int n, const T *__restrict__ x, const T *__restrict__ y,
+                            const T *__restrict__ z, double *__restrict__ out) {
+    SOFIA_PDL_ENTRY();
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 3 * n) return;
+    const int i = e / 3, d = e - 3 * i;
+    out[e] = state_value((d == 0 ? x : d == 1 ? y : z)[i]);
+}
+
 __global__ void k_fix_to_float(int n, const long long *__restrict__ fx,
                                const long long *__restrict__ fy,
                                const long long *__restrict__ fz, float *__restrict__ ff) {
@@ -2205,7 +2227,12 @@ extern "C" int sofia_force_nonbond_mixed(sofia_system *ss, const sofia_ainfo *po
     SOFIA_CUDA(ctx, s->stage_pos.ensure(pbytes));
     SOFIA_CUDA(ctx, s->stage_ff.ensure(fbytes));
     // positions (host or device) into the fixed staging buffer the graph reads
-    SOFIA_CUDA(ctx, cudaMemcpyAsync(s->stage_pos.p, position, pbytes, cudaMemcpyDefault, st));
+    sofia::HostCopies copies(ctx);
+    if (sofia::is_device_ptr(position))
+        SOFIA_CUDA(ctx, cudaMemcpyAsync(s->stage_pos.p, position, pbytes, cudaMemcpyDeviceToDevice,
+                                        st));
+    else if (const int rc = copies.in(s->stage_pos.p, position, pbytes))
+        return rc;
     const bool want_e = potential || e_coul || virial_diag3;
     const bool vir = virial_diag3 != nullptr;
     const bool graph = s->built && !s->timing;
@@ -2232,7 +2259,10 @@ extern "C" int sofia_force_nonbond_mixed(sofia_system *ss, const sofia_ainfo *po
             s->stage_ff.as<float>());
         s->launches += 2;
     }
-    SOFIA_CUDA(ctx, cudaMemcpyAsync(ff, s->stage_ff.p, fbytes, cudaMemcpyDefault, st));
+    if (sofia::is_device_ptr(ff))
+        SOFIA_CUDA(ctx, cudaMemcpyAsync(ff, s->stage_ff.p, fbytes, cudaMemcpyDeviceToDevice, st));
+    else if (const int rc = copies.out(ff, s->stage_ff.p, fbytes))
+        return rc;
     // energies and, after a graph step, the list status words come back with the
     // forces into the context's pinned buffers: one synchronization per call
     double e[5] = {0, 0, 0, 0, 0};
@@ -2243,7 +2273,7 @@ extern "C" int sofia_force_nonbond_mixed(sofia_system *ss, const sofia_ainfo *po
         SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, s->status_local.p,
                                         sizeof(int32_t) * sofia::ST_NSLOTS,
                                         cudaMemcpyDeviceToHost, st));
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
+    if (const int rc = copies.sync()) return rc;
     if (want_e) memcpy(e, ctx->h_red, sizeof(e));
     if (graph) {
         // a list row that overflowed during a device-side rebuild: grow and redo
@@ -2267,52 +2297,53 @@ extern "C" int sofia_system_set_state(sofia_system *ss, const double *x, const d
     Sys *s = &ss->s;
     sofia_nb_ctx *ctx = s->ctx;
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const size_t n = (size_t)s->n;
-    std::vector<double> h(3 * n), c(n);
+    sofia::HostCopies copies(ctx);
     const double *src[2] = {x, v};
     sofia::DevBuf *dst[2] = {s->x, s->v};
     for (int k = 0; k < 2; ++k) {
         if (!src[k]) continue;
-        SOFIA_CUDA(ctx, cudaMemcpy(h.data(), src[k], sizeof(double) * 3 * n, cudaMemcpyDefault));
-        for (int d = 0; d < 3; ++d) {
-            for (size_t i = 0; i < n; ++i) c[i] = h[3 * i + d];
-            SOFIA_CUDA(ctx, cudaMemcpy(dst[k][d].p, c.data(), sizeof(double) * n,
-                                       cudaMemcpyHostToDevice));
-        }
+        // a device array may still be written by work queued on the default stream
+        if (sofia::is_device_ptr(src[k])) SOFIA_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+        const void *in;
+        const int rc = sofia::stage_in(ctx, src[k], sizeof(double) * 3 * (size_t)s->n, k, &in);
+        if (rc) return rc;
+        sofia::launch_pdl(sofia::k_state_in, sofia::grid_for(3L * s->n, 256), 256, 0, ctx->stream,
+                          s->n, (const double *)in, dst[k][0].as<double>(),
+                          dst[k][1].as<double>(), dst[k][2].as<double>());
     }
+    SOFIA_CUDA(ctx, cudaGetLastError());
     s->built = 0;
     s->md.forces_valid = 0;
-    return SOFIA_OK;
+    return copies.sync();
 }
+
+namespace sofia {
+// The three components in atom order into the caller's [n][3] array (host or
+// device), delivered by the time of the call's sync(); stage: a staging slot.
+template <typename T>
+int state_out(Sys *s, const DevBuf (&v)[3], double *to, int stage) {
+    sofia_nb_ctx *ctx = s->ctx;
+    OutArg o;
+    if (const int rc = stage_out(ctx, to, sizeof(double) * 3 * (size_t)s->n, stage, &o)) return rc;
+    launch_pdl(k_state_out<T>, grid_for(3L * s->n, 256), 256, 0, ctx->stream, s->n, v[0].as<T>(),
+               v[1].as<T>(), v[2].as<T>(), (double *)o.dev);
+    SOFIA_CUDA(ctx, cudaGetLastError());
+    return finish_out(ctx, o);
+}
+int forces_out(Sys *s, double *f) { return state_out<long long>(s, s->f, f, 2); }
+}  // namespace sofia
 
 extern "C" int sofia_system_get_state(sofia_system *ss, double *x, double *v, double *f) {
     if (!ss) return SOFIA_EINVAL;
     Sys *s = &ss->s;
     sofia_nb_ctx *ctx = s->ctx;
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const size_t n = (size_t)s->n;
-    std::vector<double> c(n);
-    std::vector<long long> cl(n);
-    for (int d = 0; d < 3; ++d) {
-        if (x) {
-            SOFIA_CUDA(ctx, cudaMemcpy(c.data(), s->x[d].p, sizeof(double) * n,
-                                       cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < n; ++i) x[3 * i + d] = c[i];
-        }
-        if (v) {
-            SOFIA_CUDA(ctx, cudaMemcpy(c.data(), s->v[d].p, sizeof(double) * n,
-                                       cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < n; ++i) v[3 * i + d] = c[i];
-        }
-        if (f) {
-            SOFIA_CUDA(ctx, cudaMemcpy(cl.data(), s->f[d].p, sizeof(long long) * n,
-                                       cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < n; ++i) f[3 * i + d] = (double)cl[i] * sofia::FIX_INV;
-        }
-    }
-    return SOFIA_OK;
+    sofia::HostCopies copies(ctx);
+    int rc = SOFIA_OK;
+    if (x && (rc = sofia::state_out<double>(s, s->x, x, 0))) return rc;
+    if (v && (rc = sofia::state_out<double>(s, s->v, v, 1))) return rc;
+    if (f && (rc = sofia::forces_out(s, f))) return rc;
+    return copies.sync();
 }
 
 // Forces on the resident positions; energies[5] = potential, e_coul, virial x,y,z.

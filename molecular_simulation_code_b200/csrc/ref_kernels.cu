@@ -947,12 +947,12 @@ __global__ void k_add_to_float(long n, const double *__restrict__ acc, float *__
     out[i] = (float)((double)out[i] + acc[i]);
 }
 
+// Status words on the host and the call's outputs delivered.
 int check_status(sofia_nb_ctx *ctx) {
     SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status,
                                     sizeof(int32_t) * sofia::ST_NSLOTS, cudaMemcpyDeviceToHost,
                                     ctx->stream));
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return SOFIA_OK;
+    return ctx->copies->sync();
 }
 
 // Bin + sort shared by sofia_cell_sort and sofia_neighbor_build.  list: the sorted
@@ -1023,6 +1023,7 @@ extern "C" int sofia_cell_sort(sofia_nb_ctx *ctx, int np, const sofia_ainfo *pos
     if (!ctx) return SOFIA_EINVAL;
     if (np <= 0 || !position || !(box > 0.0f)) return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     const void *dpos;
     int rc = sofia::stage_in(ctx, position, sizeof(float4) * (size_t)np, 0, &dpos);
     if (rc) return rc;
@@ -1065,6 +1066,7 @@ extern "C" int sofia_neighbor_build(sofia_nb_ctx *ctx, int np, const sofia_ainfo
     if (np <= 0 || !position || !specbond || !num3bond || neigh_alloc <= 0 || !(box > 0.0f))
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     const void *dpos, *dsb, *dn3;
     int rc;
@@ -1117,11 +1119,10 @@ extern "C" int sofia_neighbor_build(sofia_nb_ctx *ctx, int np, const sofia_ainfo
         return sofia::fail(ctx, SOFIA_ENEEDGROW, "neighbour row exceeds neigh_alloc%s");
     }
     if (needed_alloc) *needed_alloc = neigh_alloc;
-    if (nlist && dlist != nlist)
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(nlist, dlist, list_bytes, cudaMemcpyDeviceToHost, st));
-    if (numneigh && dnum != numneigh)
-        SOFIA_CUDA(ctx, cudaMemcpyAsync(numneigh, dnum, sizeof(int) * (size_t)np,
-                                        cudaMemcpyDeviceToHost, st));
+    if (nlist && dlist != nlist && (rc = copies.out(nlist, dlist, list_bytes))) return rc;
+    if (numneigh && dnum != numneigh &&
+        (rc = copies.out(numneigh, dnum, sizeof(int) * (size_t)np)))
+        return rc;
     // keep the resident copy coherent when the caller's buffers were device memory
     if (dlist == nlist) {
         SOFIA_CUDA(ctx, ctx->res_nlist.ensure(list_bytes));
@@ -1133,7 +1134,7 @@ extern "C" int sofia_neighbor_build(sofia_nb_ctx *ctx, int np, const sofia_ainfo
         SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->res_numneigh.p, dnum, sizeof(int) * (size_t)np,
                                         cudaMemcpyDeviceToDevice, st));
     }
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
+    if ((rc = copies.sync())) return rc;
     return SOFIA_OK;
 }
 
@@ -1150,6 +1151,7 @@ static int force_ref_run(sofia_nb_ctx *ctx, bool long_range, int np,
     if (np <= 0 || !position || !q || !lj1 || !lj2 || !lj3 || !lj4 || ntypes <= 0 || !ff)
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dpos, *dq, *d1, *d2, *d3, *d4, *dl, *dn;
@@ -1193,7 +1195,7 @@ static int force_ref_run(sofia_nb_ctx *ctx, bool long_range, int np,
     if ((rc = sofia::finish_out(ctx, o_ff))) return rc;
     SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->h_red, ctx->red_out.p, sizeof(double) * 5,
                                     cudaMemcpyDeviceToHost, st));
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
+    if ((rc = copies.sync())) return rc;
     if (potential) *potential = ctx->h_red[0];
     if (e_coul) *e_coul = ctx->h_red[1];
     if (virial_diag3) {
@@ -1246,6 +1248,7 @@ extern "C" int sofia_pair14_dsf(sofia_nb_ctx *ctx, int np, const sofia_ainfo *po
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     if (ndihed == 0) return SOFIA_OK;
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dpos, *dq, *dlj, *ddl, *ddc;
@@ -1338,6 +1341,7 @@ extern "C" int sofia_improper_harmonic(sofia_nb_ctx *ctx, int np, const sofia_ai
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     if (nimpro == 0) return SOFIA_OK;
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dpos, *dil, *dic;
@@ -1477,6 +1481,7 @@ extern "C" int sofia_sort_gather(sofia_nb_ctx *ctx, int np, int elem_bytes, cons
         in == out)
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args (elem_bytes a multiple of 4, at most 256; in != out)%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const size_t bytes = (size_t)np * elem_bytes;
@@ -1503,6 +1508,7 @@ extern "C" int sofia_sort_specbond(sofia_nb_ctx *ctx, int np, const int32_t *tt,
     if (np <= 0 || !tt || !specbond || !num1bond || !num2bond || !num3bond)
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dt;
@@ -1532,7 +1538,7 @@ extern "C" int sofia_sort_specbond(sofia_nb_ctx *ctx, int np, const int32_t *tt,
     if ((rc = sofia::finish_out(ctx, o1))) return rc;
     if ((rc = sofia::finish_out(ctx, o2))) return rc;
     if ((rc = sofia::finish_out(ctx, o3))) return rc;
-    SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
+    if ((rc = copies.sync())) return rc;
     return SOFIA_OK;
 }
 
@@ -1544,6 +1550,7 @@ extern "C" int sofia_remap_ids(sofia_nb_ctx *ctx, int np, const int32_t *tt, int
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     if (nrows == 0 || ncols == 0) return SOFIA_OK;
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dt;
@@ -1566,6 +1573,7 @@ extern "C" int sofia_pbc(sofia_nb_ctx *ctx, int np, sofia_ainfo *position, float
     if (!ctx) return SOFIA_EINVAL;
     if (np <= 0 || !position || !(box > 0.0f)) return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     sofia::OutArg o;
@@ -1591,6 +1599,7 @@ extern "C" int sofia_correct_1x(sofia_nb_ctx *ctx, int np, const sofia_ainfo *po
         return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     if (npairs == 0) return SOFIA_OK;
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dpos, *dq, *dlist;
@@ -1761,6 +1770,7 @@ extern "C" int sofia_check_neighbor(sofia_nb_ctx *ctx, int np, const float *drx,
     if (!ctx) return SOFIA_EINVAL;
     if (np <= 0 || !drx || !dry || !drz || !nflag) return sofia::fail(ctx, SOFIA_EINVAL, "bad args%s");
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
+    sofia::HostCopies copies(ctx);
     cudaStream_t st = ctx->stream;
     int rc;
     const void *dx, *dy, *dz;

@@ -321,6 +321,9 @@ int sys_step_forces(Sys *s, int precision, bool energy, bool virial, bool force_
 // row overflowed.  status: the segment's status words already on the host, or
 // nullptr to copy them (one stream synchronization).
 int sys_list_overflow(Sys *s, const int32_t *status = nullptr);
+// The fixed-point forces as doubles into the caller's [n][3] array (host or device)
+// by the time of the call's HostCopies::sync().
+int forces_out(Sys *s, double *f);
 // Frees the captured drop-in force graphs (they bake in list pointers and the margin).
 void dropin_drop(Sys *s);
 // Column grid and list capacities for a cluster shape (mixed.cu).
