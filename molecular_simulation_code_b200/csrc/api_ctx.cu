@@ -62,6 +62,9 @@ extern "C" int sofia_nb_destroy(sofia_nb_ctx *ctx) {
     if (ctx->h_red) cudaFreeHost(ctx->h_red);
     for (auto &x : ctx->xstream)
         if (x) cudaStreamDestroy(x);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->fork) cudaEventDestroy(ctx->fork);
+    if (ctx->join) cudaEventDestroy(ctx->join);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->opened) sofia::transfer_close();
     delete ctx;

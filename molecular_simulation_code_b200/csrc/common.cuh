@@ -83,6 +83,9 @@ struct sofia_nb_ctx {
     sofia::HostCopies *copies = nullptr;                            // of the call being served
     cudaStream_t xstream[4] = {nullptr, nullptr, nullptr, nullptr};  // large host copies
     cudaStream_t stream = nullptr;
+    // a second stream for work beside the main one, joined back within a call
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     std::string last_error;
     // status words: device array + pinned host mirror
     int32_t *d_status = nullptr;

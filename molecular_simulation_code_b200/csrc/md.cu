@@ -70,10 +70,11 @@ __global__ void k_kick(int n, double h, const double *__restrict__ invm,
 // previous step's list decisions).  TWICE: the previous step's closing
 // half-kick first, as its own rounded addition (v += h f / m twice with the same
 // forces), so a segment that skips the separate closing kick gives the same bits.
-template <bool TWICE = false>
+// CLEAR: the forces, just used up, are set to zero for the step's terms to add to.
+template <bool TWICE, bool CLEAR>
 __device__ __forceinline__ void kick_drift_body(int bx, int n, double h, const double *__restrict__ invm,
-                             const long long *__restrict__ fx, const long long *__restrict__ fy,
-                             const long long *__restrict__ fz, double *__restrict__ vx,
+                             long long *__restrict__ fx, long long *__restrict__ fy,
+                             long long *__restrict__ fz, double *__restrict__ vx,
                              double *__restrict__ vy, double *__restrict__ vz, double dt,
                              double *__restrict__ x, double *__restrict__ y,
                              double *__restrict__ z, const double *__restrict__ rx,
@@ -96,6 +97,11 @@ __device__ __forceinline__ void kick_drift_body(int bx, int n, double h, const d
         ux = ux + gx;
         uy = uy + gy;
         uz = uz + gz;
+        if (CLEAR) {
+            fx[i] = 0;
+            fy[i] = 0;
+            fz[i] = 0;
+        }
         vx[i] = ux;
         vy[i] = uy;
         vz[i] = uz;
@@ -111,8 +117,8 @@ __device__ __forceinline__ void kick_drift_body(int bx, int n, double h, const d
 }
 template <bool TWICE>
 __global__ void k_kick_drift(int n, double h, const double *__restrict__ invm,
-                             const long long *__restrict__ fx, const long long *__restrict__ fy,
-                             const long long *__restrict__ fz, double *__restrict__ vx,
+                             long long *__restrict__ fx, long long *__restrict__ fy,
+                             long long *__restrict__ fz, double *__restrict__ vx,
                              double *__restrict__ vy, double *__restrict__ vz, double dt,
                              double *__restrict__ x, double *__restrict__ y,
                              double *__restrict__ z, const double *__restrict__ rx,
@@ -121,7 +127,7 @@ __global__ void k_kick_drift(int n, double h, const double *__restrict__ invm,
                              const double *__restrict__ pz, double L, double lim2, double plim2,
                              int *__restrict__ flag, long long *__restrict__ step) {
     SOFIA_PDL_ENTRY();
-    kick_drift_body<TWICE>(blockIdx.x, n, h, invm, fx, fy, fz, vx, vy, vz, dt, x, y, z, rx, ry, rz, px, py, pz, L, lim2, plim2, flag, step);
+    kick_drift_body<TWICE, true>(blockIdx.x, n, h, invm, fx, fy, fz, vx, vy, vz, dt, x, y, z, rx, ry, rz, px, py, pz, L, lim2, plim2, flag, step);
 }
 
 
@@ -784,6 +790,15 @@ static void md_dih_args(Sys *s, double *et, DihArgs *ap) {
     a.e = et + md.nbond + md.nangle;
 }
 
+// The context's second stream and its fork and join events (made before any capture).
+static cudaError_t side_open(sofia_nb_ctx *ctx) {
+    cudaError_t e = cudaSuccess;
+    if (!ctx->side) e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking);
+    for (cudaEvent_t *ev : {&ctx->fork, &ctx->join})
+        if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    return e;
+}
+
 // Parts of a step's force evaluation (all of them in an MD step; the
 // forces-only query selects).
 constexpr int MDF_PAIR = 1, MDF_LANGEVIN = 2, MDF_SHAKE = 4, MDF_ALL = 7;
@@ -808,21 +823,6 @@ static int md_forces(Sys *s, bool energy, bool force_build, bool disp_done = fal
     }
     long long *fx = s->f[0].as<long long>(), *fy = s->f[1].as<long long>(),
               *fz = s->f[2].as<long long>();
-    if (sel & MDF_PAIR) {
-        int rc = sys_step_forces(s, s->precision, energy, false, force_build, disp_done, &lg);
-        if (rc) return rc;
-    } else {
-        const size_t nb = sizeof(long long) * (size_t)s->n;
-        SOFIA_CUDA(s->ctx, cudaMemsetAsync(fx, 0, nb, st));
-        SOFIA_CUDA(s->ctx, cudaMemsetAsync(fy, 0, nb, st));
-        SOFIA_CUDA(s->ctx, cudaMemsetAsync(fz, 0, nb, st));
-        SOFIA_CUDA(s->ctx, cudaMemsetAsync(s->red.p, 0, sizeof(double) * 5, st));
-        if (lg.on) {
-            sofia::launch_pdl(k_langevin_only, grid_for(s->n, 256), 256, 0, st, s->n, lg, fx, fy,
-                              fz);
-            s->launches += 1;
-        }
-    }
     const double *x = s->x[0].as<double>(), *y = s->x[1].as<double>(), *z = s->x[2].as<double>();
     double *et = md.eterm.as<double>();
     const int nb = md.nbond, na = md.nangle, nd = md.ndihed;
@@ -844,11 +844,48 @@ static int md_forces(Sys *s, bool energy, bool force_build, bool disp_done = fal
     md_dih_args(s, et, &a);
     a.nd = b.nd;
     const long nterm = (long)b.nb + b.na + b.nd + b.ni;
-    if (nterm > 0) {
+    auto bonded = [&](cudaStream_t on) {
+        if (nterm <= 0) return;
         if (energy)
-            sofia::launch_pdl(k_bonded<true>, grid_for(nterm, 128), 128, 0, st, b);
+            sofia::launch_pdl(k_bonded<true>, grid_for(nterm, 128), 128, 0, on, b);
         else
-            sofia::launch_pdl(k_bonded<false>, grid_for(nterm, 128), 128, 0, st, b);
+            sofia::launch_pdl(k_bonded<false>, grid_for(nterm, 128), 128, 0, on, b);
+    };
+    if (disp_done) {
+        // A step: the forces were cleared with the kick, so the bonded terms need the
+        // new positions only and run beside the list maintenance and the pair kernel;
+        // the force unpack adds to their sums.  Their 10 us of latency at 9,000 atoms
+        // hide behind kernels that leave most of the GPU idle (a step 58.1 -> 51.8 us,
+        // at 37,000 atoms 120.8 -> 115.6); at 275,000 atoms the two compete and the step
+        // takes as long as before (585 and 587).
+        sofia_nb_ctx *ctx = s->ctx;
+        if (nterm > 0) {
+            SOFIA_CUDA(ctx, side_open(ctx));
+            SOFIA_CUDA(ctx, cudaEventRecord(ctx->fork, st));
+            SOFIA_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->fork, 0));
+            bonded(ctx->side);
+            SOFIA_CUDA(ctx, cudaEventRecord(ctx->join, ctx->side));
+        }
+        const int rc = sys_step_forces(s, s->precision, energy, false, force_build, true, &lg,
+                                       nullptr, nterm > 0 ? ctx->join : nullptr);
+        if (rc) return rc;
+    } else {
+        if (sel & MDF_PAIR) {
+            const int rc = sys_step_forces(s, s->precision, energy, false, force_build, false, &lg);
+            if (rc) return rc;
+        } else {
+            const size_t bytes = sizeof(long long) * (size_t)s->n;
+            SOFIA_CUDA(s->ctx, cudaMemsetAsync(fx, 0, bytes, st));
+            SOFIA_CUDA(s->ctx, cudaMemsetAsync(fy, 0, bytes, st));
+            SOFIA_CUDA(s->ctx, cudaMemsetAsync(fz, 0, bytes, st));
+            SOFIA_CUDA(s->ctx, cudaMemsetAsync(s->red.p, 0, sizeof(double) * 5, st));
+            if (lg.on) {
+                sofia::launch_pdl(k_langevin_only, grid_for(s->n, 256), 256, 0, st, s->n, lg, fx,
+                                  fy, fz);
+                s->launches += 1;
+            }
+        }
+        bonded(st);
     }
     if (md.nshake && (sel & MDF_SHAKE)) {
         sofia::launch_pdl(k_shake, grid_for(md.nshake, 128), 128, 0, st,
@@ -917,8 +954,8 @@ static int md_step(Sys *s, bool energy, bool twice = false, bool close = true) {
     const int n = s->n;
     const double h = 0.5 * md.dt * KCAL2AMU;
     double *vx = s->v[0].as<double>(), *vy = s->v[1].as<double>(), *vz = s->v[2].as<double>();
-    const long long *fx = s->f[0].as<long long>(), *fy = s->f[1].as<long long>(),
-                    *fz = s->f[2].as<long long>();
+    long long *fx = s->f[0].as<long long>(), *fy = s->f[1].as<long long>(),
+              *fz = s->f[2].as<long long>();
     const double half = 0.5 * s->skin, phalf = 0.5 * s->margin;
     sofia::launch_pdl(twice ? k_kick_drift<true> : k_kick_drift<false>, grid_for(n, 256), 256, 0, st,
         n, h, s->invm.as<double>(), fx, fy, fz, vx, vy, vz, md.dt, s->x[0].as<double>(),
@@ -959,6 +996,7 @@ static void md_drop_graphs(Sys *s) {
 
 static int md_capture(Sys *s) {
     md_drop_graphs(s);
+    SOFIA_CUDA(s->ctx, side_open(s->ctx));
     cudaStream_t st = s->ctx->stream;
     const int timing = s->timing;
     s->timing = 0;  // no event records inside the graph
@@ -1309,7 +1347,7 @@ template <bool TWICE>
 __global__ void __launch_bounds__(256, SOFIA_BATCH_STREAM_MINB) k_kick_drift_b(BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_A256)
-    kick_drift_body<TWICE>(lb, d.n, d.h, d.invm, d.fx, d.fy, d.fz, d.vx, d.vy, d.vz, d.dt, d.x, d.y,
+    kick_drift_body<TWICE, false>(lb, d.n, d.h, d.invm, d.fx, d.fy, d.fz, d.vx, d.vy, d.vz, d.dt, d.x, d.y,
                     d.z, d.rx, d.ry, d.rz, d.px, d.py, d.pz, d.L, d.lim2, d.plim2, d.flag,
                     d.step);
     SOFIA_BATCH_END

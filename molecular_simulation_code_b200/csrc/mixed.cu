@@ -1247,7 +1247,9 @@ inline cudaError_t pair_smem_optin(int nt) {
 // fixed-point range.
 // With flag != NULL, thread 0 also counts this step's list build and prune in
 // cnt and clears the trigger word for the next step's displacement check (only
-// bits are ORed into it).  With lg.on, each atom's Langevin force is added.
+// bits are ORed into it).  With lg.on, each atom's Langevin force is added.  ADD: onto
+// what the force arrays hold.
+template <bool ADD>
 __device__ __forceinline__ void unpack_body(int bx, int nslots, const int *__restrict__ ncl_dev,
                          const int *__restrict__ slot_orig, const long long *__restrict__ fslot,
                          long long *__restrict__ fx, long long *__restrict__ fy,
@@ -1272,9 +1274,15 @@ __device__ __forceinline__ void unpack_body(int bx, int nslots, const int *__res
         b += lb;
         c += lc;
     }
-    fx[o] = a;
-    fy[o] = b;
-    fz[o] = c;
+    if (ADD) {
+        fx[o] += a;
+        fy[o] += b;
+        fz[o] += c;
+    } else {
+        fx[o] = a;
+        fy[o] = b;
+        fz[o] = c;
+    }
     if (ffo) {
         ffo[3 * o + 0] = (float)((double)a * FIX_INV);
         ffo[3 * o + 1] = (float)((double)b * FIX_INV);
@@ -1284,6 +1292,7 @@ __device__ __forceinline__ void unpack_body(int bx, int nslots, const int *__res
     if (a > lim || a < -lim || b > lim || b < -lim || c > lim || c < -lim)
         atomicAdd(&status[ST_FIXED_OVF], 1);
 }
+template <bool ADD>
 __global__ void k_unpack(int nslots, const int *__restrict__ ncl_dev,
                          const int *__restrict__ slot_orig, const long long *__restrict__ fslot,
                          long long *__restrict__ fx, long long *__restrict__ fy,
@@ -1291,7 +1300,7 @@ __global__ void k_unpack(int nslots, const int *__restrict__ ncl_dev,
                          int *__restrict__ flag, long long *__restrict__ cnt, LangevinArgs lg,
                          float *__restrict__ ffo) {
     SOFIA_PDL_ENTRY();
-    unpack_body(blockIdx.x, nslots, ncl_dev, slot_orig, fslot, fx, fy, fz, status, flag, cnt, lg, ffo);
+    unpack_body<ADD>(blockIdx.x, nslots, ncl_dev, slot_orig, fslot, fx, fy, fz, status, flag, cnt, lg, ffo);
 }
 
 
@@ -1935,7 +1944,7 @@ static void launch_pair(Sys *s, int precision, bool energy, bool virial, const P
 
 // Pair kernel (+ energy reduction) on the pruned list.
 int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
-             const LangevinArgs *lg, float *ff_out) {
+             const LangevinArgs *lg, float *ff_out, cudaEvent_t join) {
     sofia_nb_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     PairConst k = make_pair_const(s, nullptr);
@@ -1957,11 +1966,18 @@ int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
               *fz = s->f[2].as<long long>();
     LangevinArgs lgv{};
     if (lg) lgv = *lg;
-    sofia::launch_pdl(k_unpack, grid_for(nslots, 256), 256, 0, st, nslots, s->nclusters.as<int>(),
-                                                    s->slot_orig.as<int>(),
-                                                    s->fslot.as<long long>(), fx, fy, fz,
-                                                    ctx->d_status, count_flag,
-                                                    s->dcount.as<long long>(), lgv, ff_out);
+    if (join) {
+        // two predecessors: a plain launch, which waits for both
+        SOFIA_CUDA(ctx, cudaStreamWaitEvent(st, join, 0));
+        k_unpack<true><<<grid_for(nslots, 256), 256, 0, st>>>(
+            nslots, s->nclusters.as<int>(), s->slot_orig.as<int>(), s->fslot.as<long long>(), fx,
+            fy, fz, ctx->d_status, count_flag, s->dcount.as<long long>(), lgv, ff_out);
+    } else {
+        sofia::launch_pdl(k_unpack<false>, grid_for(nslots, 256), 256, 0, st, nslots,
+                          s->nclusters.as<int>(), s->slot_orig.as<int>(), s->fslot.as<long long>(),
+                          fx, fy, fz, ctx->d_status, count_flag, s->dcount.as<long long>(), lgv,
+                          ff_out);
+    }
     s->launches += 2;
     if (energy || virial) {
         sofia::launch_pdl(k_red_stage1, RED_BLOCKS, 256, 0, st, s->max_clusters * ESLOT, 5, s->nclusters.as<int>(),
@@ -1980,7 +1996,7 @@ int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
 // pair kernel.  Row-capacity overflow is recorded in status_local and checked
 // by the caller after the segment (sys_list_overflow).
 int sys_step_forces(Sys *s, int precision, bool energy, bool virial, bool force_build,
-                    bool disp_done, const LangevinArgs *lg, float *ff_out) {
+                    bool disp_done, const LangevinArgs *lg, float *ff_out, cudaEvent_t join) {
     sofia_nb_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     const int n = s->n;
@@ -2001,7 +2017,7 @@ int sys_step_forces(Sys *s, int precision, bool energy, bool virial, bool force_
     sys_prune(s, flag);
     s->launches += 1;
     // the force unpack counts the build/prune events and clears the trigger word
-    return sys_pair(s, precision, energy, virial, flag, lg, ff_out);
+    return sys_pair(s, precision, energy, virial, flag, lg, ff_out, join);
 }
 
 // After a device-only segment: SOFIA_ENEEDGROW (and a larger row capacity) if
@@ -2630,7 +2646,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4) ? (EN ? SOFIA_PAIR_MINB_
 __global__ void __launch_bounds__(256, SOFIA_BATCH_STREAM_MINB) k_unpack_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_S256)
-    unpack_body(lb, d.nslots, d.ncl, d.slot_orig, reinterpret_cast<const long long *>(d.fslot),
+    unpack_body<false>(lb, d.nslots, d.ncl, d.slot_orig, reinterpret_cast<const long long *>(d.fslot),
                 d.fx, d.fy, d.fz, d.ctx_status, d.flag, d.dcount, d.lg, nullptr);
     SOFIA_BATCH_END
 }
