@@ -652,30 +652,29 @@ __global__ void k_langevin_only(int n, LangevinArgs lg, long long *__restrict__ 
     fz[i] = c;
 }
 
+__device__ __forceinline__ double ke_term(int i, const double *__restrict__ mass,
+                                          const double *__restrict__ vx,
+                                          const double *__restrict__ vy,
+                                          const double *__restrict__ vz) {
+    return 0.5 * mass[i] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]) / KCAL2AMU;
+}
 __device__ __forceinline__ void ke_body(int bx, int n, const double *__restrict__ mass, const double *__restrict__ vx,
                      const double *__restrict__ vy, const double *__restrict__ vz,
                      double *__restrict__ ke) {
     const int i = bx * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    ke[i] = 0.5 * mass[i] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]) / KCAL2AMU;
+    if (i < n) ke[i] = ke_term(i, mass, vx, vy, vz);
 }
-__global__ void k_ke(int n, const double *__restrict__ mass, const double *__restrict__ vx,
-                     const double *__restrict__ vy, const double *__restrict__ vz,
-                     double *__restrict__ ke) {
-    SOFIA_PDL_ENTRY();
-    ke_body(blockIdx.x, n, mass, vx, vy, vz, ke);
-}
-
-
-// Two-stage deterministic sum of column c of in[n][w] into out[slot].
+// Two-stage deterministic sum of n terms.
 constexpr int MRED = 64;
-__device__ __forceinline__ void mred1_body(int bx, int n, int w, int c, const double *__restrict__ in,
-                        double *__restrict__ part, int nblk) {
+static_assert(MRED == 64 && MD_NJOB <= 8, "k_md_energy: two partials per lane, a warp per job");
+template <class Term>
+__device__ __forceinline__ void mred1_body(int bx, int n, double *__restrict__ part, int nblk,
+                                           Term term) {
     __shared__ double s[256];
     const int chunk = (n + nblk - 1) / nblk;
     const int b0 = bx * chunk, b1 = min(n, b0 + chunk);
     double acc = 0.0;
-    for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) acc += in[(size_t)i * w + c];
+    for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) acc += term(i);
     s[threadIdx.x] = acc;
     __syncthreads();
     for (int off = 128; off > 0; off >>= 1) {
@@ -683,11 +682,6 @@ __device__ __forceinline__ void mred1_body(int bx, int n, int w, int c, const do
         __syncthreads();
     }
     if (threadIdx.x == 0) part[bx] = s[0];
-}
-__global__ void k_mred1(int n, int w, int c, const double *__restrict__ in,
-                        double *__restrict__ part) {
-    SOFIA_PDL_ENTRY();
-    mred1_body(blockIdx.x, n, w, c, in, part, (int)gridDim.x);
 }
 __device__ __forceinline__ void mred2_body(int bx, const double *__restrict__ part, double *__restrict__ out) {
     __shared__ double s[MRED];
@@ -699,22 +693,51 @@ __device__ __forceinline__ void mred2_body(int bx, const double *__restrict__ pa
     }
     if (threadIdx.x == 0) out[0] = s[0];
 }
-__global__ void k_mred2(const double *__restrict__ part, double *__restrict__ out) {
+// All energy sums of a step in one launch: MRED blocks per job sum contiguous ranges,
+// the block that finishes last sums every job's partials (warp j takes job j, in the
+// order of mred2_body) and copies the pair sums.  done wraps to zero with the last
+// block.  As two launches per job plus the kinetic terms they took 16 launches, about
+// 35 us at the end of a run.
+struct EnergyJobs {
+    int n[MD_NJOB], w[MD_NJOB], c[MD_NJOB], slot[MD_NJOB];  // n = 0: off
+    const double *in[MD_NJOB];
+    int kin;  // the job whose terms are the kinetic energies of n atoms
+    const double *mass, *vx, *vy, *vz;
+    const double *pair;  // five pair sums, to slots 0..4
+    double *part, *out;
+    unsigned *done;
+};
+__global__ void __launch_bounds__(256) k_md_energy(EnergyJobs e) {
     SOFIA_PDL_ENTRY();
-    mred2_body(blockIdx.x, part, out);
+    const int job = blockIdx.x / MRED, blk = blockIdx.x - job * MRED;
+    if (e.n[job] > 0) {
+        if (job == e.kin)
+            mred1_body(blk, e.n[job], e.part + job * MRED, MRED,
+                       [&](int i) { return ke_term(i, e.mass, e.vx, e.vy, e.vz); });
+        else
+            mred1_body(blk, e.n[job], e.part + job * MRED, MRED,
+                       [&](int i) { return e.in[job][(size_t)i * e.w[job] + e.c[job]]; });
+    }
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(e.done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+    if (j < MD_NJOB && e.n[j] > 0) {
+        double v = __ldcg(e.part + j * MRED + lane) + __ldcg(e.part + j * MRED + lane + 32);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0) e.out[e.slot[j]] = v;
+    }
+    if (threadIdx.x < 5) e.out[threadIdx.x] = e.pair[threadIdx.x];
 }
 
 }  // namespace
 
-static void md_reduce(cudaStream_t st, int n, int w, int c, const double *in, double *part,
-                      double *out) {
-    if (n <= 0) return;
-    sofia::launch_pdl(k_mred1, MRED, 256, 0, st, n, w, c, in, part);
-    sofia::launch_pdl(k_mred2, 1, MRED, 0, st, part, out);
-}
-
 // energies slots in md.ered: 0 lj, 1 coul, (2..4 pair virial), 5 bond, 6 angle,
-// 7 torsion, 8 coul14, 9 lj14, 10 kinetic; partials after slot 16.
+// 7 torsion, 8 coul14, 9 lj14, 10 kinetic, 11 improper.
 // All bonded terms of a step in one launch: threads [0, nb) take bonds, the
 // next na angles, then nd dihedrals (torsion and 1-4 pair), then ni impropers.
 // A count of 0 switches a term off.
@@ -900,28 +923,34 @@ static int md_forces(Sys *s, bool energy, bool force_build, bool disp_done = fal
 
 static void md_energy_reduce(Sys *s) {
     Md &md = s->md;
-    cudaStream_t st = s->ctx->stream;
-    double *red = md.ered.as<double>();
-    double *part = red + 16;
     double *et = md.eterm.as<double>();
-    // nonbonded pair energies were reduced into s->red by the pair path
-    cudaMemcpyAsync(red, s->red.p, sizeof(double) * 5, cudaMemcpyDeviceToDevice, st);  // checked with the step's launches
-    if (md.nbond && (md.terms & 1)) md_reduce(st, md.nbond, 1, 0, et, part, red + 5);
-    if (md.nangle && (md.terms & 2)) md_reduce(st, md.nangle, 1, 0, et + md.nbond, part, red + 6);
-    if (md.ndihed && (md.terms & 12)) {
-        const double *ed = et + md.nbond + md.nangle;
-        md_reduce(st, md.ndihed, 3, 0, ed, part, red + 7);
-        md_reduce(st, md.ndihed, 3, 1, ed, part, red + 8);
-        md_reduce(st, md.ndihed, 3, 2, ed, part, red + 9);
+    const int nb = md.nbond, na = md.nangle, nd = md.ndihed;
+    const int dn = (md.terms & 12) ? nd : 0;
+    const double *ed = et + nb + na;
+    const double *ein[MD_NJOB] = {et, et + nb, ed, ed, ed, ed + 3 * (size_t)nd, nullptr};
+    const int n[MD_NJOB] = {(md.terms & 1) ? nb : 0, (md.terms & 2) ? na : 0, dn, dn, dn,
+                            (md.terms & 16) ? md.nimpro : 0, s->n};
+    const int w[MD_NJOB] = {1, 1, 3, 3, 3, 1, 1}, c[MD_NJOB] = {0, 0, 0, 1, 2, 0, 0};
+    const int slot[MD_NJOB] = {5, 6, 7, 8, 9, 11, 10};
+    EnergyJobs e;
+    for (int j = 0; j < MD_NJOB; ++j) {
+        e.n[j] = n[j];
+        e.w[j] = w[j];
+        e.c[j] = c[j];
+        e.slot[j] = slot[j];
+        e.in[j] = ein[j];
     }
-    if (md.nimpro && (md.terms & 16))
-        md_reduce(st, md.nimpro, 1, 0, et + md.nbond + md.nangle + 3 * (size_t)md.ndihed, part,
-                  red + 11);
-    double *ke = md.eterm.as<double>() + (md.nbond + md.nangle + 3 * (size_t)md.ndihed +
-                                          (size_t)md.nimpro);
-    sofia::launch_pdl(k_ke, grid_for(s->n, 256), 256, 0, st, s->n, s->mass.as<double>(), s->v[0].as<double>(),
-                                              s->v[1].as<double>(), s->v[2].as<double>(), ke);
-    md_reduce(st, s->n, 1, 0, ke, part, red + 10);
+    e.kin = MD_NJOB - 1;
+    e.mass = s->mass.as<double>();
+    e.vx = s->v[0].as<double>();
+    e.vy = s->v[1].as<double>();
+    e.vz = s->v[2].as<double>();
+    e.pair = s->red.as<double>();
+    e.part = md.bpart.as<double>();
+    e.out = md.ered.as<double>();
+    e.done = reinterpret_cast<unsigned *>(md.ered.as<double>() + 16);
+    sofia::launch_pdl(k_md_energy, MD_NJOB * MRED, 256, 0, s->ctx->stream, e);
+    s->launches += 1;
 }
 
 // Reduced device energies (red slots: 0-1 pair, 5 bond, 6 angle, 7-9 torsion,
@@ -1111,9 +1140,9 @@ extern "C" int sofia_system_md_setup(sofia_system *ss, const sofia_md_desc *d) {
     const size_t nterm = (size_t)md.nbond + md.nangle + 3 * (size_t)md.ndihed +
                          (size_t)md.nimpro + (size_t)s->n;
     SOFIA_CUDA(ctx, md.eterm.ensure(sizeof(double) * nterm));
-    SOFIA_CUDA(ctx, md.ered.ensure(sizeof(double) * (16 + sofia::MRED)));
+    SOFIA_CUDA(ctx, md.ered.ensure(sizeof(double) * 17));  // sums, k_md_energy's counter
     SOFIA_CUDA(ctx, md.bpart.ensure(sizeof(double) * sofia::MD_NJOB * sofia::MRED));
-    SOFIA_CUDA(ctx, cudaMemset(md.ered.p, 0, sizeof(double) * 16));
+    SOFIA_CUDA(ctx, cudaMemset(md.ered.p, 0, sizeof(double) * 17));
     SOFIA_CUDA(ctx, md.step_dev.ensure(sizeof(long long)));
     SOFIA_CUDA(ctx, cudaMemset(md.step_dev.p, 0, sizeof(long long)));
     for (int k = 0; k < 6; ++k) SOFIA_CUDA(ctx, md.snap[k].ensure(sizeof(double) * s->n));
@@ -1410,8 +1439,9 @@ __global__ void k_mred1_b(const BatchDev *__restrict__ tab) {
     SOFIA_BATCH_LOOP(BK_MRED)
     const int job = lb / MRED, blk = lb - job * MRED;
     if (d.job_n[job] > 0)
-        mred1_body(blk, d.job_n[job], d.job_w[job], d.job_c[job], d.job_in[job],
-                   d.ebpart + job * MRED, MRED);
+        mred1_body(blk, d.job_n[job], d.ebpart + job * MRED, MRED, [&](int i) {
+            return d.job_in[job][(size_t)i * d.job_w[job] + d.job_c[job]];
+        });
     __syncthreads();
     SOFIA_BATCH_END
 }

@@ -1452,51 +1452,60 @@ __global__ void k_set_flag(int *__restrict__ flag, int v) {
     if (threadIdx.x == 0 && blockIdx.x == 0) flag[0] = v;
 }
 
-// Two-stage deterministic column sums: stage 1 = fixed grid of blocks over
-// contiguous ranges (coalesced), stage 2 = one block over the partials.
-// n rows at most, ESLOT per cluster of ncl_dev.
-__device__ __forceinline__ void red_stage1_body(int bx, int n, int w, const int *__restrict__ ncl_dev,
+// Deterministic sums of the pair kernel's five energy columns: RED_BLOCKS blocks sum
+// contiguous ranges of rows (n at most, ESLOT per cluster of ncl_dev), then the
+// blocks' partials are summed in block order.  All columns go through one pass and
+// one barrier per stage.
+constexpr int NE = 5;
+__device__ __forceinline__ void red_stage1_body(int bx, int n, const int *__restrict__ ncl_dev,
                              const double *__restrict__ in, double *__restrict__ part, int nblk) {
-    __shared__ double s[256];
+    __shared__ double s[8][NE];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nn = min(n, ncl_dev[0] * ESLOT);
     const int chunk = (nn + nblk - 1) / nblk;
     const int b0 = bx * chunk, b1 = min(nn, b0 + chunk);
-    for (int c = 0; c < w; ++c) {
-        double acc = 0.0;
-        for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) acc += in[(size_t)i * w + c];
-        s[threadIdx.x] = acc;
-        __syncthreads();
-        for (int off = 128; off > 0; off >>= 1) {
-            if (threadIdx.x < off) s[threadIdx.x] += s[threadIdx.x + off];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) part[bx * w + c] = s[0];
-        __syncthreads();
+    double acc[NE] = {};
+    for (int i = b0 + threadIdx.x; i < b1; i += 256)
+#pragma unroll
+        for (int c = 0; c < NE; ++c) acc[c] += in[(size_t)i * NE + c];
+#pragma unroll
+    for (int c = 0; c < NE; ++c) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) acc[c] += __shfl_xor_sync(FULL, acc[c], off);
+        if (lane == 0) s[w][c] = acc[c];
+    }
+    __syncthreads();
+    if (threadIdx.x < NE) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += s[k][threadIdx.x];
+        part[bx * NE + threadIdx.x] = v;
     }
 }
-__global__ void k_red_stage1(int n, int w, const int *__restrict__ ncl_dev,
-                             const double *__restrict__ in, double *__restrict__ part) {
-    SOFIA_PDL_ENTRY();
-    red_stage1_body(blockIdx.x, n, w, ncl_dev, in, part, (int)gridDim.x);
+// Warp c sums column c of the partials.
+__device__ __forceinline__ void red_stage2_body(int nblk, const double *part,
+                                                double *__restrict__ out) {
+    const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+    if (c >= NE) return;
+    double v = 0.0;
+    for (int k = lane; k < nblk; k += 32) v += __ldcg(part + k * NE + c);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
+    if (lane == 0) out[c] = v;
 }
-__device__ __forceinline__ void red_stage2_body(int bx, int nblk, int w, const double *__restrict__ part,
-                             double *__restrict__ out, double scale) {
-    __shared__ double s[256];
-    for (int c = 0; c < w; ++c) {
-        s[threadIdx.x] = (threadIdx.x < nblk) ? part[threadIdx.x * w + c] : 0.0;
-        __syncthreads();
-        for (int off = 128; off > 0; off >>= 1) {
-            if (threadIdx.x < off) s[threadIdx.x] += s[threadIdx.x + off];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[c] = scale * s[0];
-        __syncthreads();
-    }
-}
-__global__ void k_red_stage2(int nblk, int w, const double *__restrict__ part,
-                             double *__restrict__ out, double scale) {
+// Both stages in one launch: the block that finishes last takes the second.  done
+// counts the finished blocks and wraps to zero with the last one.
+__global__ void __launch_bounds__(256) k_red(int n, const int *__restrict__ ncl_dev,
+                                             const double *__restrict__ in, double *part,
+                                             double *__restrict__ out, unsigned *done) {
     SOFIA_PDL_ENTRY();
-    red_stage2_body(blockIdx.x, nblk, w, part, out, scale);
+    red_stage1_body(blockIdx.x, n, ncl_dev, in, part, (int)gridDim.x);
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) red_stage2_body((int)gridDim.x, part, out);
 }
 
 // Ballistic drift x += dt*v (FP64), used to move a system between
@@ -1512,15 +1521,33 @@ __global__ void k_drift(int n, double dt, double *__restrict__ x, double *__rest
     z[i] += dt * vz[i];
 }
 
+// Reference records -> FP64 SoA positions; with flag, also the displacement triggers
+// (as k_disp_check) on the positions just read.
+template <bool TRIGGER>
 __global__ void k_aos_to_soa(int n, const float4 *__restrict__ pos, double *__restrict__ x,
-                             double *__restrict__ y, double *__restrict__ z) {
+                             double *__restrict__ y, double *__restrict__ z,
+                             const double *__restrict__ rx, const double *__restrict__ ry,
+                             const double *__restrict__ rz, const double *__restrict__ px,
+                             const double *__restrict__ py, const double *__restrict__ pz,
+                             double L, double lim2, double plim2, int *__restrict__ flag) {
     SOFIA_PDL_ENTRY();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pos[i];
-    x[i] = (double)p.x;
-    y[i] = (double)p.y;
-    z[i] = (double)p.z;
+    bool far = false, pfar = false;
+    if (i < n) {
+        const float4 p = pos[i];
+        const double a = (double)p.x, b = (double)p.y, c = (double)p.z;
+        x[i] = a;
+        y[i] = b;
+        z[i] = c;
+        if (TRIGGER) {
+            far = disp2(a, b, c, rx[i], ry[i], rz[i], L) > lim2;
+            pfar = disp2(a, b, c, px[i], py[i], pz[i], L) > plim2;
+        }
+    }
+    if (TRIGGER) {
+        const bool a = __any_sync(FULL, far), b = __any_sync(FULL, pfar);
+        if ((threadIdx.x & 31) == 0 && (a || b)) atomicOr(flag, (a ? 1 : 0) | (b ? 2 : 0));
+    }
 }
 
 // The caller's [n][3] state arrays <-> the SoA state.  One thread per value: the
@@ -1596,8 +1623,10 @@ static int sys_alloc(Sys *s) {
     for (int d = 0; d < 3; ++d) SOFIA_CUDA(ctx, s->xprn[d].ensure(sizeof(double) * n));
     SOFIA_CUDA(ctx, s->icount.ensure(sizeof(int) * maxcl));
     SOFIA_CUDA(ctx, s->part.ensure(sizeof(double) * 8 * RED_BLOCKS));
+    SOFIA_CUDA(ctx, cudaMemset(s->part.p, 0, sizeof(double) * 8 * RED_BLOCKS));  // k_red's counter
     SOFIA_CUDA(ctx, s->dcount.ensure(sizeof(long long) * 4));
     SOFIA_CUDA(ctx, cudaMemset(s->dcount.p, 0, sizeof(long long) * 4));
+    SOFIA_CUDA(ctx, cudaMemset(s->flag.p, 0, sizeof(int) * 4));
     SOFIA_CUDA(ctx, cudaMemset(s->status_local.p, 0, sizeof(int) * ST_NSLOTS));
     // no clusters and empty rows until the first build (host queries may come first)
     SOFIA_CUDA(ctx, cudaMemset(s->nclusters.p, 0, sizeof(int) * 4));
@@ -1850,6 +1879,8 @@ int sys_eval(Sys *s, int precision, bool energy, bool virial, bool force_build) 
         SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
         build = (h & 1) != 0;
         prune = h != 0;
+        // whoever ORs into the trigger word next finds it cleared
+        SOFIA_CUDA(ctx, cudaMemsetAsync(s->flag.p, 0, sizeof(int), st));
     }
     if (s->timing) sys_collect_timers(s);
     for (int attempt = 0; attempt < 4; ++attempt) {
@@ -1980,12 +2011,12 @@ int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
     }
     s->launches += 2;
     if (energy || virial) {
-        sofia::launch_pdl(k_red_stage1, RED_BLOCKS, 256, 0, st, s->max_clusters * ESLOT, 5, s->nclusters.as<int>(),
-                                                 s->energy.as<double>(), s->part.as<double>());
         // the half list holds each pair once: no halving
-        sofia::launch_pdl(k_red_stage2, 1, 256, 0, st, RED_BLOCKS, 5, s->part.as<double>(), s->red.as<double>(),
-                                        1.0);
-        s->launches += 2;
+        sofia::launch_pdl(k_red, RED_BLOCKS, 256, 0, st, s->max_clusters * ESLOT,
+                          s->nclusters.as<int>(), s->energy.as<double>(), s->part.as<double>(),
+                          s->red.as<double>(),
+                          reinterpret_cast<unsigned *>(s->part.as<double>() + NE * RED_BLOCKS));
+        s->launches += 1;
     }
     SOFIA_CUDA(ctx, cudaGetLastError());
     return SOFIA_OK;
@@ -2044,6 +2075,18 @@ int sys_list_overflow(Sys *s, const int32_t *status) {
     return SOFIA_OK;
 }
 
+// The staged reference records into the resident positions; TRIGGER: with the list
+// triggers, ORed into the trigger word that the last evaluation left cleared.
+template <bool TRIGGER>
+static void dropin_positions(Sys *s) {
+    const double half = 0.5 * s->skin, phalf = 0.5 * s->margin;
+    launch_pdl(k_aos_to_soa<TRIGGER>, grid_for(s->n, 256), 256, 0, s->ctx->stream, s->n,
+               s->stage_pos.as<float4>(), s->x[0].as<double>(), s->x[1].as<double>(),
+               s->x[2].as<double>(), s->xref[0].as<double>(), s->xref[1].as<double>(),
+               s->xref[2].as<double>(), s->xprn[0].as<double>(), s->xprn[1].as<double>(),
+               s->xprn[2].as<double>(), s->L, half * half, phalf * phalf, s->flag.as<int>());
+}
+
 // The drop-in force call as one CUDA graph: AoS positions -> FP64 SoA,
 // displacement triggers, conditional rebuild and prune, pair kernel, forces ->
 // real*4 AoS.  It reads stage_pos and writes stage_ff; variant e: 0 forces,
@@ -2057,11 +2100,9 @@ static int dropin_capture(Sys *s, int e) {
     const long long l0 = s->launches;
     cudaGraph_t g = nullptr;
     SOFIA_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    sofia::launch_pdl(k_aos_to_soa, grid_for(n, 256), 256, 0, st, n, s->stage_pos.as<float4>(),
-                                                   s->x[0].as<double>(), s->x[1].as<double>(),
-                                                   s->x[2].as<double>());
+    dropin_positions<true>(s);
     // the force unpack also writes the real*4 forces the call returns
-    const int rc = sys_step_forces(s, s->precision, e >= 1, e == 2, false, false, nullptr,
+    const int rc = sys_step_forces(s, s->precision, e >= 1, e == 2, false, true, nullptr,
                                    s->stage_ff.as<float>());
     const cudaError_t ce = cudaStreamEndCapture(st, &g);
     s->dropin_launches[e] = s->launches - l0 + 1;
@@ -2265,9 +2306,7 @@ extern "C" int sofia_force_nonbond_mixed(sofia_system *ss, const sofia_ainfo *po
         s->launches += s->dropin_launches[e];
     } else {
         // first call after creation or set_state (or with timers on): host-driven
-        sofia::launch_pdl(sofia::k_aos_to_soa, sofia::grid_for(n, 256), 256, 0, st,
-            n, s->stage_pos.as<float4>(), s->x[0].as<double>(), s->x[1].as<double>(),
-            s->x[2].as<double>());
+        sofia::dropin_positions<false>(s);
         const int rc = sofia::sys_eval(s, s->precision, want_e, vir, false);
         if (rc) return rc;
         sofia::launch_pdl(sofia::k_fix_to_float, sofia::grid_for(n, 256), 256, 0, st,
@@ -2654,7 +2693,7 @@ __global__ void __launch_bounds__(256, SOFIA_BATCH_STREAM_MINB) k_unpack_b(const
 __global__ void k_red_stage1_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_RED)
-    red_stage1_body(lb, d.maxcl * ESLOT, 5, d.ncl, d.energy, d.part, RED_BLOCKS);
+    red_stage1_body(lb, d.maxcl * ESLOT, d.ncl, d.energy, d.part, RED_BLOCKS);
     __syncthreads();
     SOFIA_BATCH_END
 }
@@ -2662,7 +2701,7 @@ __global__ void k_red_stage1_b(const BatchDev *__restrict__ tab) {
 __global__ void k_red_stage2_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_REP)
-    red_stage2_body(lb, RED_BLOCKS, 5, d.part, d.red, 1.0);
+    red_stage2_body(RED_BLOCKS, d.part, d.red);
     __syncthreads();
     SOFIA_BATCH_END
 }
