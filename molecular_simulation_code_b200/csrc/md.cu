@@ -1719,12 +1719,11 @@ static int batch_capture(sofia_batch *b) {
         cudaGraphDestroy(graph);
         if (ce != cudaSuccess) return sofia::cuda_fail(ctx, ce, "cudaGraphInstantiate (batch)");
     }
-    // a step: kick+drift, the pair path (active-replica compaction, bin, scan,
-    // scatter, sort, pack with the cluster boxes, search, prune, pair, unpack),
-    // bonded, SHAKE; then the closing kick (+ RATTLE), once per segment when the
+    // a step: kick+drift, the pair path (active-replica compaction, bin, scan, sort,
+    // pack with the cluster boxes, search, prune, pair, unpack), bonded, SHAKE; then the closing kick (+ RATTLE), once per segment when the
     // kicks are chained; energies add the two pair-energy and four MD-energy
     // reductions
-    const long long body = 1 + 10 + 2, closing = 1 + (rat ? 1 : 0);
+    const long long body = 1 + 9 + 2, closing = 1 + (rat ? 1 : 0);
     b->graph_launches[0] = body + closing;
     b->graph_launches[1] = body + closing + 6;
     b->graph_launches[2] = rat ? b->seg * (body + closing) : b->seg * body + closing;
@@ -2011,7 +2010,7 @@ extern "C" int sofia_system_device_bytes(sofia_system *ss, int64_t *bytes) {
         &s->x[0], &s->x[1], &s->x[2], &s->v[0], &s->v[1], &s->v[2], &s->f[0], &s->f[1], &s->f[2],
         &s->xref[0], &s->xref[1], &s->xref[2], &s->img[0], &s->img[1], &s->img[2], &s->type,
         &s->q, &s->invm, &s->mass, &s->specbond, &s->num3bond, &s->ljtab, &s->col_count,
-        &s->col_start, &s->col_fill, &s->col_atoms, &s->col_key, &s->cl_start, &s->slot_orig,
+        &s->col_start, &s->bucket, &s->cl_start, &s->slot_orig,
         &s->rec, &s->bb, &s->jlist, &s->jmask, &s->jcount, &s->nclusters, &s->recf, &s->fslot,
         &s->atom_slot, &s->status_local, &s->energy, &s->red, &s->flag, &s->stage_pos,
         &s->stage_ff, &s->cl_pos, &s->cl_gid, &s->ptta, &s->ilist, &s->imask, &s->icount,

@@ -93,15 +93,16 @@ __device__ __forceinline__ double wrap_shift(double x, double L) {
     return -L * floor(x / L);
 }
 
-__device__ __forceinline__ void wrap_bin_body(int bx, const int *__restrict__ cond, int cmask, int n,
+// Wraps every atom, keeps its position and wrap shift, and drops its sort key into
+// its xy column's bucket.
+__device__ __forceinline__ void wrap_bin_body(int bx, int n,
                            const double *__restrict__ x, const double *__restrict__ y,
                            const double *__restrict__ z, double L, double s_col, int ncx,
                            double *__restrict__ ix, double *__restrict__ iy,
                            double *__restrict__ iz, double *__restrict__ rx,
                            double *__restrict__ ry, double *__restrict__ rz,
-                           int *__restrict__ col_of, int *__restrict__ col_count,
-                           float *__restrict__ zkey) {
-    SOFIA_COND_RETURN;
+                           int *__restrict__ col_count,
+                           unsigned long long *__restrict__ bucket) {
     int i = bx * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double px = x[i], py = y[i], pz = z[i];
@@ -122,121 +123,102 @@ __device__ __forceinline__ void wrap_bin_body(int bx, const int *__restrict__ co
     cx = max(cx, 0);
     cy = max(cy, 0);
     const int c = cx + cy * ncx;
-    col_of[i] = c;
-    zkey[i] = (float)wz;
-    atomicAdd(&col_count[c], 1);
+    // sort key: z, then index; an overfull column's surplus is dropped and reported
+    // by the column sort
+    const int at = atomicAdd(&col_count[c], 1);
+    const unsigned zb = __float_as_uint(fmaxf((float)wz, 0.0f));
+    if (at < MAX_COL)
+        bucket[(size_t)c * MAX_COL + at] = ((unsigned long long)zb << 32) | (unsigned)i;
 }
-__global__ void k_wrap_bin(const int *__restrict__ cond, int cmask, int n,
-                           const double *__restrict__ x, const double *__restrict__ y,
-                           const double *__restrict__ z, double L, double s_col, int ncx,
-                           double *__restrict__ ix, double *__restrict__ iy,
-                           double *__restrict__ iz, double *__restrict__ rx,
-                           double *__restrict__ ry, double *__restrict__ rz,
-                           int *__restrict__ col_of, int *__restrict__ col_count,
-                           float *__restrict__ zkey) {
-    SOFIA_PDL_ENTRY();
-    wrap_bin_body(blockIdx.x, cond, cmask, n, x, y, z, L, s_col, ncx, ix, iy, iz, rx, ry, rz, col_of, col_count, zkey);
-}
-
-// Column scans of a build, one block: col_start = exclusive scan of the atom
-// counts, cl_start = exclusive scan of the cluster counts (ceil(count/8)), the
-// total cluster count into ncl.  The counts are cleared for the next build.
-__device__ __forceinline__ void scan_cols_body(int bx, const int *__restrict__ cond, int cmask, int n,
-                            int *__restrict__ col_count, int *__restrict__ col_start,
-                            int *__restrict__ cl_start, int *__restrict__ ncl) {
-    SOFIA_COND_RETURN;
-    __shared__ int s1[1024], s2[1024];
-    __shared__ int carry1, carry2;
-    const int t = threadIdx.x;
-    if (t == 0) carry1 = carry2 = 0;
-    __syncthreads();
-    for (int base = 0; base < n; base += 1024) {
-        const int v = (base + t < n) ? col_count[base + t] : 0;
-        const int w = (v + CL - 1) / CL;
-        s1[t] = v;
-        s2[t] = w;
+// Column scans of a build, by one block: col_start = exclusive scan of the atom
+// counts, cl_start = exclusive scan of the cluster counts (ceil(count/8)), the total
+// cluster count into ncl.  The counts are cleared for the next build.
+__device__ __forceinline__ void scan_cols_body(int n, int *col_count, int *__restrict__ col_start,
+                                               int *__restrict__ cl_start, int *__restrict__ ncl) {
+    __shared__ int2 s_w[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
+    int2 carry = make_int2(0, 0);
+    for (int base = 0; base < n; base += blockDim.x) {
+        const int v = (base + t < n) ? __ldcg(col_count + base + t) : 0;
+        const int u = (v + CL - 1) / CL;
+        int2 incl = make_int2(v, u);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int a = __shfl_up_sync(FULL, incl.x, off), b = __shfl_up_sync(FULL, incl.y, off);
+            if (lane >= off) {
+                incl.x += a;
+                incl.y += b;
+            }
+        }
+        if (lane == 31) s_w[w] = incl;
         __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            const int a1 = (t >= off) ? s1[t - off] : 0;
-            const int a2 = (t >= off) ? s2[t - off] : 0;
-            __syncthreads();
-            s1[t] += a1;
-            s2[t] += a2;
-            __syncthreads();
+        int2 before = carry, total = make_int2(0, 0);
+        for (int k = 0; k < nw; ++k) {
+            const int2 x = s_w[k];
+            if (k < w) {
+                before.x += x.x;
+                before.y += x.y;
+            }
+            total.x += x.x;
+            total.y += x.y;
         }
         if (base + t < n) {
-            col_start[base + t] = carry1 + s1[t] - v;
-            cl_start[base + t] = carry2 + s2[t] - w;
+            col_start[base + t] = before.x + incl.x - v;
+            cl_start[base + t] = before.y + incl.y - u;
             col_count[base + t] = 0;
         }
-        __syncthreads();
-        if (t == 1023) {
-            carry1 += s1[1023];
-            carry2 += s2[1023];
-        }
+        carry.x += total.x;
+        carry.y += total.y;
         __syncthreads();
     }
     if (t == 0) {
-        col_start[n] = carry1;
-        cl_start[n] = carry2;
-        ncl[0] = carry2;
+        col_start[n] = carry.x;
+        cl_start[n] = carry.y;
+        ncl[0] = carry.y;
     }
 }
-__global__ void k_scan_cols(const int *__restrict__ cond, int cmask, int n,
-                            int *__restrict__ col_count, int *__restrict__ col_start,
-                            int *__restrict__ cl_start, int *__restrict__ ncl) {
-    SOFIA_PDL_ENTRY();
-    scan_cols_body(blockIdx.x, cond, cmask, n, col_count, col_start, cl_start, ncl);
-}
 
-__device__ __forceinline__ void col_scatter_body(int bx, const int *__restrict__ cond, int cmask, int n,
-                              const int *__restrict__ col_of,
-                              const int *__restrict__ col_start, int *__restrict__ col_fill,
-                              int *__restrict__ col_atoms) {
-    SOFIA_COND_RETURN;
-    int i = bx * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int c = col_of[i];
-    const int s = atomicAdd(&col_fill[c], 1);
-    col_atoms[col_start[c] + s] = i;
-}
-__global__ void k_col_scatter(const int *__restrict__ cond, int cmask, int n,
-                              const int *__restrict__ col_of,
-                              const int *__restrict__ col_start, int *__restrict__ col_fill,
-                              int *__restrict__ col_atoms) {
+// Binning and, by the block that finishes last, the column scans (done counts the
+// finished blocks and wraps to zero).  A step launches the build kernels whether or
+// not it builds, so each one fewer is a microsecond of every step.
+__global__ void __launch_bounds__(256) k_wrap_bin(
+    const int *__restrict__ cond, int cmask, int n, const double *__restrict__ x,
+    const double *__restrict__ y, const double *__restrict__ z, double L, double s_col, int ncx,
+    double *__restrict__ ix, double *__restrict__ iy, double *__restrict__ iz,
+    double *__restrict__ rx, double *__restrict__ ry, double *__restrict__ rz,
+    int *__restrict__ col_count, unsigned long long *__restrict__ bucket, int ncols,
+    int *__restrict__ col_start, int *__restrict__ cl_start, int *__restrict__ ncl,
+    unsigned *__restrict__ done) {
     SOFIA_PDL_ENTRY();
-    col_scatter_body(blockIdx.x, cond, cmask, n, col_of, col_start, col_fill, col_atoms);
+    SOFIA_COND_RETURN;
+    wrap_bin_body(blockIdx.x, n, x, y, z, L, s_col, ncx, ix, iy, iz, rx, ry, rz, col_count, bucket);
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) scan_cols_body(ncols, col_count, col_start, cl_start, ncl);
 }
 
 // Sort each column by (z, index); then lay the column out as clusters of 8.
-__device__ __forceinline__ void col_sort_assign_body(int bx, const int *__restrict__ cond, int cmask, int ncols,
+__device__ __forceinline__ void col_sort_assign_body(int bx, int ncols,
                                   const int *__restrict__ col_start,
-                                  int *__restrict__ col_atoms, const float *__restrict__ zkey,
+                                  const unsigned long long *__restrict__ bucket,
                                   const int *__restrict__ cl_start, int *__restrict__ slot_orig,
                                   int *__restrict__ cl_col, int *__restrict__ atom_slot,
-                                  int *__restrict__ col_fill, int *__restrict__ status) {
-    SOFIA_COND_RETURN;
+                                  int *__restrict__ status) {
     __shared__ unsigned long long s[MAX_COL];
     const int c = bx;
     if (c >= ncols) return;
-    // the scatter is done with this column's fill counter: clear it for the next build
-    if (threadIdx.x == 0) col_fill[c] = 0;
-    const int b = col_start[c], nc = col_start[c + 1] - b;
+    const int nc = col_start[c + 1] - col_start[c];
     if (nc > MAX_COL) {
         if (threadIdx.x == 0) atomicAdd(&status[ST_CELLOVER], 1);
         return;
     }
     int m = 1;
     while (m < nc) m <<= 1;
-    for (int t = threadIdx.x; t < m; t += blockDim.x) {
-        if (t < nc) {
-            const int i = col_atoms[b + t];
-            const unsigned zb = __float_as_uint(fmaxf(zkey[i], 0.0f));
-            s[t] = ((unsigned long long)zb << 32) | (unsigned)i;
-        } else {
-            s[t] = ~0ull;
-        }
-    }
+    for (int t = threadIdx.x; t < m; t += blockDim.x)
+        s[t] = t < nc ? bucket[(size_t)c * MAX_COL + t] : ~0ull;
     __syncthreads();
     for (int k = 2; k <= m; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
@@ -262,14 +244,15 @@ __device__ __forceinline__ void col_sort_assign_body(int bx, const int *__restri
         if ((t & (CL - 1)) == 0) cl_col[c0 + t / CL] = c;
     }
 }
-__global__ void k_col_sort_assign(const int *__restrict__ cond, int cmask, int ncols,
-                                  const int *__restrict__ col_start,
-                                  int *__restrict__ col_atoms, const float *__restrict__ zkey,
-                                  const int *__restrict__ cl_start, int *__restrict__ slot_orig,
-                                  int *__restrict__ cl_col, int *__restrict__ atom_slot,
-                                  int *__restrict__ col_fill, int *__restrict__ status) {
+__global__ void __launch_bounds__(256) k_col_sort_assign(
+    const int *__restrict__ cond, int cmask, int ncols, const int *__restrict__ col_start,
+    const unsigned long long *__restrict__ bucket, const int *__restrict__ cl_start,
+    int *__restrict__ slot_orig, int *__restrict__ cl_col, int *__restrict__ atom_slot,
+    int *__restrict__ status) {
     SOFIA_PDL_ENTRY();
-    col_sort_assign_body(blockIdx.x, cond, cmask, ncols, col_start, col_atoms, zkey, cl_start, slot_orig, cl_col, atom_slot, col_fill, status);
+    SOFIA_COND_RETURN;
+    col_sort_assign_body(blockIdx.x, ncols, col_start, bucket, cl_start, slot_orig, cl_col,
+                         atom_slot, status);
 }
 
 // Gather the cluster-ordered records.  The position used is the build-time
@@ -1600,12 +1583,9 @@ static int sys_alloc(Sys *s) {
     }
     SOFIA_CUDA(ctx, s->col_count.ensure(sizeof(int) * (s->ncols + 1)));
     SOFIA_CUDA(ctx, s->col_start.ensure(sizeof(int) * (s->ncols + 1)));
-    SOFIA_CUDA(ctx, s->col_fill.ensure(sizeof(int) * (s->ncols + 1)));
     SOFIA_CUDA(ctx, cudaMemset(s->col_count.p, 0, sizeof(int) * (s->ncols + 1)));
-    SOFIA_CUDA(ctx, cudaMemset(s->col_fill.p, 0, sizeof(int) * (s->ncols + 1)));
     SOFIA_CUDA(ctx, s->cl_start.ensure(sizeof(int) * (s->ncols + 1)));
-    SOFIA_CUDA(ctx, s->col_atoms.ensure(sizeof(int) * n * 2));  // atoms + column of atom
-    SOFIA_CUDA(ctx, s->col_key.ensure(sizeof(float) * n));
+    SOFIA_CUDA(ctx, s->bucket.ensure(sizeof(unsigned long long) * MAX_COL * (size_t)s->ncols));
     const size_t maxcl = (size_t)s->max_clusters;
     SOFIA_CUDA(ctx, s->slot_orig.ensure(sizeof(int) * maxcl * CL + sizeof(int) * maxcl));
     SOFIA_CUDA(ctx, s->rec.ensure(sizeof(ClusterRec) * maxcl));
@@ -1632,6 +1612,8 @@ static int sys_alloc(Sys *s) {
     SOFIA_CUDA(ctx, cudaMemset(s->nclusters.p, 0, sizeof(int) * 4));
     SOFIA_CUDA(ctx, cudaMemset(s->jcount.p, 0, sizeof(int) * maxcl));
     SOFIA_CUDA(ctx, cudaMemset(s->icount.p, 0, sizeof(int) * maxcl));
+    // the context's stream does not wait for these by itself
+    SOFIA_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
     return SOFIA_OK;
 }
 
@@ -1699,27 +1681,21 @@ static void sys_build_bin(Sys *s, const int *cond) {
     cudaStream_t st = ctx->stream;
     const int n = s->n;
     const int cm = 1;
-    int *col_of = s->col_atoms.as<int>() + n;
     int *cl_col = s->slot_orig.as<int>() + (size_t)s->max_clusters * CL;
-    // col_count and col_fill start at zero (set at creation, cleared after each
-    // use); every slot of the new clusters is written by the column sort
+    // col_count starts at zero (set at creation, cleared by the scans); every slot of
+    // the new clusters is written by the column sort
     sofia::launch_pdl(k_wrap_bin, grid_for(n, 256), 256, 0, st,
         cond, cm, n, s->x[0].as<double>(), s->x[1].as<double>(), s->x[2].as<double>(), s->L,
         s->s_col, s->ncx, s->img[0].as<double>(), s->img[1].as<double>(), s->img[2].as<double>(),
-        s->xref[0].as<double>(), s->xref[1].as<double>(), s->xref[2].as<double>(), col_of,
-        s->col_count.as<int>(), s->col_key.as<float>());
-    sofia::launch_pdl(k_scan_cols, 1, 1024, 0, st, cond, cm, s->ncols, s->col_count.as<int>(),
-                                    s->col_start.as<int>(), s->cl_start.as<int>(),
-                                    s->nclusters.as<int>());
-    sofia::launch_pdl(k_col_scatter, grid_for(n, 256), 256, 0, st, cond, cm, n, col_of, s->col_start.as<int>(),
-                                                    s->col_fill.as<int>(),
-                                                    s->col_atoms.as<int>());
-    sofia::launch_pdl(k_col_sort_assign, s->ncols, 256, 0, st, cond, cm, s->ncols, s->col_start.as<int>(),
-                                                s->col_atoms.as<int>(), s->col_key.as<float>(),
-                                                s->cl_start.as<int>(), s->slot_orig.as<int>(),
-                                                cl_col, s->atom_slot.as<int>(),
-                                                s->col_fill.as<int>(), s->status_local.as<int>());
-    s->launches += 4;
+        s->xref[0].as<double>(), s->xref[1].as<double>(), s->xref[2].as<double>(),
+        s->col_count.as<int>(), s->bucket.as<unsigned long long>(), s->ncols,
+        s->col_start.as<int>(), s->cl_start.as<int>(), s->nclusters.as<int>(),
+        reinterpret_cast<unsigned *>(s->nclusters.as<int>() + 1));
+    sofia::launch_pdl(k_col_sort_assign, s->ncols, 256, 0, st, cond, cm, s->ncols,
+                      s->col_start.as<int>(), s->bucket.as<unsigned long long>(),
+                      s->cl_start.as<int>(), s->slot_orig.as<int>(), cl_col,
+                      s->atom_slot.as<int>(), s->status_local.as<int>());
+    s->launches += 2;
 }
 
 // Part 2: cluster bounding boxes and the cluster-pair search.
@@ -2242,8 +2218,7 @@ extern "C" int sofia_system_destroy(sofia_system *ss) {
     s->icount.release();
     s->part.release();
     sofia::DevBuf *bufs[] = {&s->type, &s->q, &s->invm, &s->mass, &s->specbond, &s->num3bond,
-                             &s->ljtab, &s->col_count, &s->col_start, &s->col_fill, &s->col_atoms,
-                             &s->col_key, &s->cl_start, &s->slot_orig, &s->rec, &s->bb, &s->jlist,
+                             &s->ljtab, &s->col_count, &s->col_start, &s->bucket, &s->cl_start, &s->slot_orig, &s->rec, &s->bb, &s->jlist,
                              &s->jmask, &s->jcount, &s->nclusters, &s->status_local, &s->energy,
                              &s->red, &s->flag, &s->stage_pos, &s->stage_ff, &s->cl_pos,
                              &s->cl_gid, &s->ptta};
@@ -2584,31 +2559,24 @@ namespace {
 __global__ void k_wrap_bin_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_ACTIVE_LOOP(BK_A256, BA_BUILD)
-    wrap_bin_body(lb, d.flag, 1, d.n, d.x, d.y, d.z, d.L, d.s_col, d.ncx, d.ix, d.iy, d.iz, d.rx,
-                  d.ry, d.rz, d.col_of, d.col_count, d.col_key);
+    wrap_bin_body(lb, d.n, d.x, d.y, d.z, d.L, d.s_col, d.ncx, d.ix, d.iy, d.iz, d.rx, d.ry, d.rz,
+                  d.col_count, d.bucket);
     SOFIA_BATCH_END
 }
 
 __global__ void __launch_bounds__(1024) k_scan_cols_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_ACTIVE_LOOP(BK_SCAN, BA_BUILD)
-    scan_cols_body(lb, d.flag, 1, d.ncols, d.col_count, d.col_start, d.cl_start, d.ncl);
+    scan_cols_body(d.ncols, d.col_count, d.col_start, d.cl_start, d.ncl);
     __syncthreads();
-    SOFIA_BATCH_END
-}
-
-__global__ void k_col_scatter_b(const BatchDev *__restrict__ tab) {
-    SOFIA_PDL_ENTRY();
-    SOFIA_BATCH_ACTIVE_LOOP(BK_A256, BA_BUILD)
-    col_scatter_body(lb, d.flag, 1, d.n, d.col_of, d.col_start, d.col_fill, d.col_atoms);
     SOFIA_BATCH_END
 }
 
 __global__ void k_col_sort_assign_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_ACTIVE_LOOP(BK_COLS, BA_BUILD)
-    col_sort_assign_body(lb, d.flag, 1, d.ncols, d.col_start, d.col_atoms, d.col_key, d.cl_start,
-                         d.slot_orig, d.cl_col, d.atom_slot, d.col_fill, d.status);
+    col_sort_assign_body(lb, d.ncols, d.col_start, d.bucket, d.cl_start, d.slot_orig, d.cl_col,
+                         d.atom_slot, d.status);
     __syncthreads();
     SOFIA_BATCH_END
 }
@@ -2819,14 +2787,11 @@ void repdev_fill_pair(const Sys *s, RepDev *d) {
     d->num3bond = s->num3bond.as<int>();
     d->col_count = s->col_count.as<int>();
     d->col_start = s->col_start.as<int>();
-    d->col_fill = s->col_fill.as<int>();
-    d->col_atoms = s->col_atoms.as<int>();
-    d->col_of = s->col_atoms.as<int>() + s->n;
+    d->bucket = s->bucket.as<unsigned long long>();
     d->cl_start = s->cl_start.as<int>();
     d->slot_orig = s->slot_orig.as<int>();
     d->cl_col = s->slot_orig.as<int>() + (size_t)s->max_clusters * CL;
     d->atom_slot = s->atom_slot.as<int>();
-    d->col_key = s->col_key.as<float>();
     d->rec = s->rec.as<ClusterRec>();
     d->sref = s->sref.as<double>();
     d->recf = s->recf.as<float>();
@@ -2873,7 +2838,6 @@ void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
     launch_pdl(k_batch_active_b, 1, MAXREP, 0, st, tab);
     launch_pdl(k_wrap_bin_b, g256, 256, 0, st, tab);
     launch_pdl(k_scan_cols_b, nsm * 2, 1024, 0, st, tab);
-    launch_pdl(k_col_scatter_b, g256, 256, 0, st, tab);
     launch_pdl(k_col_sort_assign_b, nsm * 4, 256, 0, st, tab);
     launch_pdl(k_pack_b, g256, 256, 0, st, tab);
     // one block per warp-per-cluster virtual block of all members (blocks past the

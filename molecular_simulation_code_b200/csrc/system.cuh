@@ -91,7 +91,8 @@ struct Sys {
     DevBuf type, q, invm, mass, specbond, num3bond;
     DevBuf ljtab;                      // float4 {lj1,lj2,lj3,lj4} per type pair
     // cluster structures
-    DevBuf col_count, col_start, col_fill, col_atoms, col_key, cl_start;
+    DevBuf col_count, col_start, cl_start;
+    DevBuf bucket;                      // sort keys per column, MAX_COL places each
     DevBuf slot_orig, rec, bb, jlist, jmask, jcount, nclusters;
     DevBuf recf;                        // FP32 positions per cluster: x[8], y[8], z[8]
     DevBuf fslot;                       // pair forces in cluster-slot order, 64-bit fixed point [3][slots]
@@ -199,9 +200,8 @@ struct RepDev {
     const float *q;
     const int *type, *specbond, *num3bond;
     // list build and cluster order
-    int *col_count, *col_start, *col_fill, *col_atoms, *col_of, *cl_start, *slot_orig, *cl_col,
-        *atom_slot;
-    float *col_key;
+    int *col_count, *col_start, *cl_start, *slot_orig, *cl_col, *atom_slot;
+    unsigned long long *bucket;
     ClusterRec *rec;
     double *sref;
     float *recf;
