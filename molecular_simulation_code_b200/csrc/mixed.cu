@@ -1299,6 +1299,10 @@ __global__ void k_unpack(int nslots, const int *__restrict__ ncl_dev,
 // or ballots.  Distances here only select
 // pairs, so FP32 copies of the positions suffice (the squared radius carries a
 // 1e-3 A^2 safety margin).
+// SPLIT warps share a row: in each round warp `part` takes the part-th of the next
+// SPLIT x 32 entries and learns from the others' counts where its survivors go, so
+// the pruned row is the same for every SPLIT.
+template <int SPLIT>
 __device__ __forceinline__ void prune_body(int bx, 
     const int *__restrict__ cond, int cmask, int maxcl, const int *__restrict__ ncl_dev,
     const float *__restrict__ recf,
@@ -1317,12 +1321,14 @@ __device__ __forceinline__ void prune_body(int bx,
         s_shf[im * 3 + 1] = (float)((im / 3) % 3 - 1) * L;
         s_shf[im * 3 + 2] = (float)(im / 9 - 1) * L;
     }
+    __shared__ int s_cnt[2][8];  // survivors per warp, by round parity
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int icl = (bx * blockDim.x + threadIdx.x) >> 5;
+    const int wid = (bx * blockDim.x + threadIdx.x) >> 5;
+    const int icl = wid / SPLIT, part = wid % SPLIT;
     if (icl >= maxcl || icl >= ncl_dev[0]) return;
     // the positions this prune is valid for (the prune trigger measures from them)
-    if (lane < CL) {
+    if (part == 0 && lane < CL) {
         const int o = slot_orig[icl * CL + lane];
         if (o >= 0) {
             px[o] = x[o];
@@ -1347,8 +1353,8 @@ __device__ __forceinline__ void prune_body(int bx,
     int *orow = ilist + (size_t)icl * jcap;
     unsigned long long *omrow = imask + (size_t)icl * jcap;
     int kept = 0;
-    for (int base = 0; base < n; base += 32) {
-        const int e = base + lane;
+    for (int base = 0, round = 0; base < n; base += 32 * SPLIT, ++round) {
+        const int e = base + 32 * part + lane;
         const bool active = e < n;
         const int w = active ? row[e] : 0;
         const unsigned long long m = active ? mrow[e] : 0ull;
@@ -1405,15 +1411,30 @@ __device__ __forceinline__ void prune_body(int bx,
         const unsigned long long newm = (((unsigned long long)hi << 32) | lo) & m;
         const bool keep = newm != 0ull;
         const unsigned kb = __ballot_sync(FULL, keep);
+        int before = 0, all = __popc(kb);
+        if (SPLIT > 1) {
+            // one barrier of the row's warps per round: the counts alternate
+            const int w0 = (threadIdx.x >> 5) - part;
+            int *cnt = s_cnt[round & 1] + w0;
+            if (lane == 0) cnt[part] = all;
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + w0 / SPLIT), "n"(32 * SPLIT) : "memory");
+            all = 0;
+#pragma unroll
+            for (int k = 0; k < SPLIT; ++k) {
+                if (k < part) before += cnt[k];
+                all += cnt[k];
+            }
+        }
         if (keep) {
-            const int at = kept + __popc(kb & ((1u << lane) - 1u));
+            const int at = kept + before + __popc(kb & ((1u << lane) - 1u));
             orow[at] = w;
             omrow[at] = newm;
         }
-        kept += __popc(kb);
+        kept += all;
     }
-    if (lane == 0) icount[icl] = kept;
+    if (part == 0 && lane == 0) icount[icl] = kept;
 }
+template <int SPLIT>
 __global__ void __launch_bounds__(256, SOFIA_PRUNE_MINB) k_prune(
     const int *__restrict__ cond, int cmask, int maxcl, const int *__restrict__ ncl_dev,
     const float *__restrict__ recf,
@@ -1425,7 +1446,7 @@ __global__ void __launch_bounds__(256, SOFIA_PRUNE_MINB) k_prune(
     const double *__restrict__ y, const double *__restrict__ z, double *__restrict__ px,
     double *__restrict__ py, double *__restrict__ pz) {
     SOFIA_PDL_ENTRY();
-    prune_body(blockIdx.x, cond, cmask, maxcl, ncl_dev, recf, jlist, jmask, jcount, jcap, L, rin2, rfar2, bb, ilist, imask, icount, slot_orig, x, y, z, px, py, pz);
+    prune_body<SPLIT>(blockIdx.x, cond, cmask, maxcl, ncl_dev, recf, jlist, jmask, jcount, jcap, L, rin2, rfar2, bb, ilist, imask, icount, slot_orig, x, y, z, px, py, pz);
 }
 
 
@@ -1812,6 +1833,17 @@ static PairConst make_pair_const(const Sys *s, const float *lj_dummy) {
     return k;
 }
 
+// Clusters of a system (half of a column's last cluster is empty on average).
+static long expected_rows(const Sys *s) { return s->n / CL + s->ncols / 2; }
+
+// Warps per list row of the prune: 4 while 4 per row are resident at once, where a row
+// of 130 outer entries is a serial chain on a GPU that is mostly idle (MD us per step at
+// 1 / 4: 3,000 atoms 45.3 / 44.3, 9,000 51.1 / 50.1, 16,000 67.5 / 68.8, 275,000 584 /
+// 622: the rounds' barriers cost more than they hide once the warps fill the GPU).
+static int prune_split(const Sys *s) {
+    return 4 * expected_rows(s) <= (long)s->nsm * 32 ? 4 : 1;
+}
+
 // Launches: displacement check, conditional rebuild, pack, pair kernel.
 // `force_build` rebuilds regardless of the trigger.
 // The cluster boxes come from the record pack that precedes every prune.
@@ -1820,8 +1852,9 @@ static void sys_prune(Sys *s, const int *cond) {
     const float rin = (float)(s->rc + s->margin);
     const float rin2 = rin * rin + 1e-3f;
     const float rfar = rin + 0.01f;
-    sofia::launch_pdl(k_prune, grid_for((long)s->max_clusters * 32, 256), 256, 0, st,
-        cond, 3, s->max_clusters, s->nclusters.as<int>(), s->recf.as<float>(),
+    const int split = prune_split(s);
+    sofia::launch_pdl(split == 4 ? k_prune<4> : k_prune<1>,
+        grid_for((long)s->max_clusters * 32 * split, 256), 256, 0, st, cond, 3, s->max_clusters, s->nclusters.as<int>(), s->recf.as<float>(),
         s->jlist.as<int>(), s->jmask.as<unsigned long long>(), s->jcount.as<int>(), s->jcap,
         (float)s->L, rin2, rfar * rfar, s->bb.as<float4>(), s->ilist.as<int>(),
         s->imask.as<unsigned long long>(),
@@ -1905,9 +1938,8 @@ static int pair_split(const Sys *s, int precision) {
     // the table of this many types allows one block less per SM: one warp per row
     if (pair_smem(s->ntypes, false, true) > 32768) return 1;
     const bool mixed = precision != SOFIA_PREC_FP64;
-    // resident warps, and the rows (half of a column's last cluster is empty on average)
-    const long res = (long)s->nsm * (mixed ? 32 : 16);
-    const long rows = s->n / CL + s->ncols / 2;
+    const long res = (long)s->nsm * (mixed ? 32 : 16);  // resident warps
+    const long rows = expected_rows(s);
     if (4 * rows <= res) return 4;
     return (mixed ? rows : 2 * rows) <= res ? 2 : 1;
 }
@@ -2632,7 +2664,7 @@ __global__ void __launch_bounds__(256, SOFIA_BATCH_SEARCH_MINB) k_search_b(Batch
 __global__ void __launch_bounds__(256, SOFIA_PRUNE_MINB) k_prune_b(BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_ACTIVE_LOOP(BK_W256, BA_PRUNE)
-    prune_body(lb, d.flag, 3, d.maxcl, d.ncl, d.recf, d.jlist, d.jmask, d.jcount, d.jcap,
+    prune_body<1>(lb, d.flag, 3, d.maxcl, d.ncl, d.recf, d.jlist, d.jmask, d.jcount, d.jcap,
                (float)d.L, d.rin2, d.rfar2, d.bb, d.ilist, d.imask, d.icount, d.slot_orig, d.x,
                d.y, d.z, d.px, d.py, d.pz);
     __syncthreads();
