@@ -638,8 +638,8 @@ struct PairConst {
     float ljs6;
     float2 ljs6_2;
     double ljs6d;
-    double rcut2d, cut_coulsqd, alphad, e_shiftd, f_shiftd, coulpred, MY_PIS_INV;
-    double A1d, A2d, A3d, A4d, A5d, EWALD_Pd;
+    double rcut2d, cut_coulsqd, kexpd, pad, c2ad, e_shiftd, f_shiftd;
+    double A1d, A2d, A3d, A4d, A5d;
     double L;
     int ntypes;
 };
@@ -713,37 +713,33 @@ struct PairMath<float> {
     }
 };
 
+// FP64 pair: the same forms.  The FP64 pipe bounds this kernel, so the pair takes one
+// reciprocal square root for 1/r, 1/r^2 and r instead of a square root and two
+// divisions, and fused multiply-adds instead of separate products and sums.
 template <>
 struct PairMath<double> {
     template <bool EN, bool SAME>
     __device__ __forceinline__ static double eval(double dx, double dy, double dz, double qiq,
                                                   float4 lj, bool on, const PairConst &k,
                                                   double &elj, double &ec) {
-        // the reference's expressions and order, each operation rounded on its own
-        const double r2 = addr(addr(mulr(dx, dx), mulr(dy, dy)), mulr(dz, dz));
-        const double r = sqrt(r2);
-        const double rinv = 1.0 / r;
-        const double r2inv = 1.0 / r2;
+        const double r2 = fmar(dx, dx, fmar(dy, dy, mulr(dz, dz)));
+        const double rinv = rsqrt(r2);
+        const double r2inv = mulr(rinv, rinv);
+        const double r = r2 == 0.0 ? 0.0 : mulr(r2, rinv);  // 0, not 0 * inf
         const double dr6i = mulr(mulr(r2inv, r2inv), r2inv);
         const bool lj_on = on && r2 <= k.rcut2d;
         const bool c_on = on && r2 <= k.cut_coulsqd;
-        const double flj = mulr(dr6i, addr(mulr((double)lj.x, dr6i), -(double)lj.y));
+        const double flj = mulr(dr6i, fmar((double)lj.x, dr6i, -(double)lj.y));
         const double pref = mulr(qiq, rinv);
-        const double ex = exp(-mulr(mulr(mulr(k.alphad, k.alphad), r), r));
-        const double t = 1.0 / addr(1.0, mulr(mulr(k.EWALD_Pd, k.alphad), r));
-        const double poly = addr(k.A1d, mulr(t, addr(k.A2d, mulr(t, addr(k.A3d,
-                            mulr(t, addr(k.A4d, mulr(t, k.A5d))))))));
+        const double ex = exp(mulr(k.kexpd, r2));
+        const double t = 1.0 / fmar(k.pad, r, 1.0);
+        const double poly = fmar(t, fmar(t, fmar(t, fmar(t, k.A5d, k.A4d), k.A3d), k.A2d), k.A1d);
         const double erfcc = mulr(mulr(t, poly), ex);
-        const double c2a = mulr(mulr(2.0, k.alphad), k.MY_PIS_INV);
-        const double fc = mulr(mulr(pref, addr(addr(mulr(erfcc, rinv), mulr(c2a, ex)),
-                                               mulr(r, k.f_shiftd))), r);
+        const double fc = mulr(pref, fmar(k.f_shiftd, r2, fmar(mulr(k.c2ad, ex), r, erfcc)));
         if (EN) {
-            const double esh = mulr(k.ljs6d, addr(mulr(k.ljs6d, (double)lj.z), -(double)lj.w));
-            elj = lj_on ? addr(mulr(dr6i, addr(mulr(dr6i, (double)lj.z), -(double)lj.w)), -esh)
-                        : 0.0;
-            ec = c_on ? mulr(pref, addr(addr(erfcc, -mulr(r, k.e_shiftd)),
-                                        -mulr(r2, k.f_shiftd)))
-                      : 0.0;
+            const double esh = mulr(k.ljs6d, fmar(k.ljs6d, (double)lj.z, -(double)lj.w));
+            elj = lj_on ? addr(mulr(dr6i, fmar(dr6i, (double)lj.z, -(double)lj.w)), -esh) : 0.0;
+            ec = c_on ? mulr(pref, fmar(-k.f_shiftd, r2, fmar(-k.e_shiftd, r, erfcc))) : 0.0;
         }
         const double fs = mulr(addr(c_on ? fc : 0.0, lj_on ? flj : 0.0), r2inv);
         return on ? fs : 0.0;
@@ -1791,20 +1787,19 @@ static PairConst make_pair_const(const Sys *s, const float *lj_dummy) {
     k.cut_coulsqd = rcut2;
     k.rcut2 = (float)rcut2;
     k.cut_coulsq = (float)rcut2;
-    k.alphad = s->alpha;
+    k.kexpd = -(s->alpha * s->alpha);
     k.kexp = (float)(-(s->alpha * s->alpha) * 1.4426950408889634);  // -alpha^2 log2(e)
     const double EP = (double)0.3275911f;
-    k.EWALD_Pd = EP;
+    k.pad = EP * s->alpha;
     k.pa = (float)(EP * s->alpha);
     const double mypis = (double)1.77245385090551602729f;
-    k.MY_PIS_INV = 1.0 / mypis;
+    k.c2ad = (2.0 * s->alpha) / mypis;
     k.c2a = (float)((2.0 * s->alpha) / mypis);
     k.e_shiftd = s->e_shift;
     k.f_shiftd = s->f_shift;
     k.e_shift = (float)s->e_shift;
     k.f_shift = (float)s->f_shift;
     k.coulpre = s->coulpre;
-    k.coulpred = (double)s->coulpre;
     k.A1d = (double)0.254829592f;
     k.A2d = (double)-0.284496736f;
     k.A3d = (double)1.421413741f;
