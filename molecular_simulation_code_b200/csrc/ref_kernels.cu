@@ -521,6 +521,7 @@ __global__ void __launch_bounds__(256) k_force_ref(
     const float *__restrict__ lj4, int ntypes, const int *__restrict__ nlist,
     const int *__restrict__ numneigh, int neigh_alloc, DsfConst k, float *__restrict__ ff,
     double *__restrict__ pe) {
+    SOFIA_PDL_ENTRY();
     __shared__ int s_queue[8][SWEEP_QUEUE];
     const int lane = threadIdx.x & 31;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -624,6 +625,7 @@ __global__ void __launch_bounds__(256) k_force_long_ref(
     const float *__restrict__ lj4, int ntypes, const int *__restrict__ nlist,
     const int *__restrict__ numneigh, int neigh_alloc, DsfConst k, float *__restrict__ ff,
     double *__restrict__ pe) {
+    SOFIA_PDL_ENTRY();
     __shared__ int s_queue[8][SWEEP_QUEUE];
     const int lane = threadIdx.x & 31;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -704,48 +706,60 @@ __global__ void __launch_bounds__(256) k_force_long_ref(
     }
 }
 
-// Fixed-order reduction of per-item partials pe[n][w] -> out[w]: a fixed grid
-// of blocks sums contiguous ranges (coalesced), then one block sums the
-// partials, so the result does not depend on scheduling.
+// Fixed-order reduction of per-item partials pe[n][W] -> scale * sums: a fixed grid of
+// blocks sums contiguous ranges (coalesced, all columns in one pass) and the block that
+// finishes last sums the blocks' partials (warp c takes column c), so the result does
+// not depend on scheduling.  done counts the finished blocks and wraps to zero.
 constexpr int RED_BLOCKS = 128;
-__global__ void k_red1(int n, int w, const double *__restrict__ pe, double *__restrict__ part) {
-    __shared__ double s[256];
+constexpr int RED_DOUBLES = 16 + 8 * RED_BLOCKS;  // sums, the counter (at 8), partials (from 16)
+template <int W>
+__global__ void __launch_bounds__(256) k_red(int n, const double *__restrict__ pe, double *part,
+                                             double *__restrict__ out, double scale,
+                                             unsigned *done) {
+    SOFIA_PDL_ENTRY();
+    __shared__ double s[8][W];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int chunk = (n + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
-    for (int c = 0; c < w; ++c) {
-        double acc = 0.0;
-        for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) acc += pe[(size_t)i * w + c];
-        s[threadIdx.x] = acc;
-        __syncthreads();
-        for (int off = 128; off > 0; off >>= 1) {
-            if (threadIdx.x < off) s[threadIdx.x] += s[threadIdx.x + off];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) part[blockIdx.x * w + c] = s[0];
-        __syncthreads();
+    double acc[W] = {};
+    for (int i = b0 + threadIdx.x; i < b1; i += 256)
+#pragma unroll
+        for (int c = 0; c < W; ++c) acc[c] += pe[(size_t)i * W + c];
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+        const double v = warp_sum(acc[c]);
+        if (lane == 0) s[w][c] = v;
     }
-}
-__global__ void k_red2(int w, const double *__restrict__ part, double *__restrict__ out,
-                       double scale) {
-    __shared__ double s[256];
-    for (int c = 0; c < w; ++c) {
-        s[threadIdx.x] = (threadIdx.x < RED_BLOCKS) ? part[threadIdx.x * w + c] : 0.0;
-        __syncthreads();
-        for (int off = 128; off > 0; off >>= 1) {
-            if (threadIdx.x < off) s[threadIdx.x] += s[threadIdx.x + off];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[c] = scale * s[0];
-        __syncthreads();
+    __syncthreads();
+    if (threadIdx.x < W) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += s[k][threadIdx.x];
+        part[blockIdx.x * W + threadIdx.x] = v;
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last || w >= W) return;
+    double v = 0.0;
+    for (int k = lane; k < (int)gridDim.x; k += 32) v += __ldcg(part + k * W + w);
+    v = warp_sum(v);
+    if (lane == 0) out[w] = scale * v;
 }
 
-// pe[n][w] -> out[w] (out = red_out, partials after it)
-inline void reduce_cols(cudaStream_t st, int n, int w, const double *pe, double *out,
-                        double scale) {
-    double *part = out + 16;
-    k_red1<<<RED_BLOCKS, 256, 0, st>>>(n, w, pe, part);
-    k_red2<<<1, 256, 0, st>>>(w, part, out, scale);
+// pe[n][W] -> out[W]; out has RED_DOUBLES, the counter among them zero before the first call
+template <int W>
+inline void reduce_cols(cudaStream_t st, int n, const double *pe, double *out, double scale) {
+    sofia::launch_pdl(k_red<W>, RED_BLOCKS, 256, 0, st, n, pe, out + 16, out, scale,
+                      reinterpret_cast<unsigned *>(out + 8));
+}
+inline int reduce_room(sofia_nb_ctx *ctx) {
+    if (ctx->red_out.p) return SOFIA_OK;
+    SOFIA_CUDA(ctx, ctx->red_out.ensure(sizeof(double) * RED_DOUBLES));
+    SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->red_out.p, 0, sizeof(double) * RED_DOUBLES, ctx->stream));
+    return SOFIA_OK;
 }
 
 // Minimum image of mod_minimg.f90:5-15: d - box*nint(ibox*d), box*nint() in real*4.
@@ -762,6 +776,7 @@ __global__ void k_dihedral_dsf(int ndihed, int np, const float4 *__restrict__ po
                                const double *__restrict__ dc, int ndtypes, DsfConst k, float box,
                                float ibox, double *__restrict__ acc, double *__restrict__ pe,
                                int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= ndihed) return;
     const int i1 = dl[n * 5] - 1, i2 = dl[n * 5 + 1] - 1, i3 = dl[n * 5 + 2] - 1,
@@ -899,6 +914,7 @@ __global__ void k_correct_pairs(int npairs, int np, const float4 *__restrict__ p
                                 int stride, int ca, int cb, DsfConst k, double gewald,
                                 double fudge, float coulpre, double *__restrict__ acc,
                                 double *__restrict__ pe, int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= npairs) return;
     const int i1 = list[(size_t)m * stride + ca] - 1, i2 = list[(size_t)m * stride + cb] - 1;
@@ -942,6 +958,7 @@ __global__ void k_correct_pairs(int npairs, int np, const float4 *__restrict__ p
 
 // out[i] = (float)((double)in[i] + acc[i]) for the float force arrays the reference adds into.
 __global__ void k_add_to_float(long n, const double *__restrict__ acc, float *__restrict__ out) {
+    SOFIA_PDL_ENTRY();
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     out[i] = (float)((double)out[i] + acc[i]);
@@ -1178,10 +1195,10 @@ static int force_ref_run(sofia_nb_ctx *ctx, bool long_range, int np,
     sofia::OutArg o_ff;
     if ((rc = sofia::stage_out(ctx, ff, sizeof(float) * 3 * (size_t)np, 8, &o_ff))) return rc;
     SOFIA_CUDA(ctx, ctx->pe_atom.ensure(sizeof(double) * 5 * (size_t)np));
-    SOFIA_CUDA(ctx, ctx->red_out.ensure(sizeof(double) * (16 + 8 * RED_BLOCKS)));
+    if ((rc = reduce_room(ctx))) return rc;
     const long threads = (long)np * 32;
     if (long_range)
-        k_force_long_ref<<<sofia::grid_for(threads, 256), 256, 0, st>>>(
+        sofia::launch_pdl(k_force_long_ref, sofia::grid_for(threads, 256), 256, 0, st,
             np, (const float4 *)dpos, (const float *)dq, (const float *)d1, (const float *)d2,
             (const float *)d3, (const float *)d4, ntypes, (const int *)dl, (const int *)dn,
             neigh_alloc, k, (float *)o_ff.dev, ctx->pe_atom.as<double>());
@@ -1190,7 +1207,7 @@ static int force_ref_run(sofia_nb_ctx *ctx, bool long_range, int np,
             np, (const float4 *)dpos, (const float *)dq, (const float *)d1, (const float *)d2,
             (const float *)d3, (const float *)d4, ntypes, (const int *)dl, (const int *)dn,
             neigh_alloc, k, (float *)o_ff.dev, ctx->pe_atom.as<double>());
-    reduce_cols(st, np, 5, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 0.5);
+    reduce_cols<5>(st, np, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 0.5);
     SOFIA_CUDA(ctx, cudaGetLastError());
     if ((rc = sofia::finish_out(ctx, o_ff))) return rc;
     SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->h_red, ctx->red_out.p, sizeof(double) * 5,
@@ -1263,16 +1280,16 @@ extern "C" int sofia_pair14_dsf(sofia_nb_ctx *ctx, int np, const sofia_ainfo *po
     if ((rc = sofia::stage_out(ctx, ffh, sizeof(float) * 3 * (size_t)np, 5, &o_ff, true))) return rc;
     SOFIA_CUDA(ctx, ctx->acc64.ensure(sizeof(double) * 3 * (size_t)np));
     SOFIA_CUDA(ctx, ctx->pe_atom.ensure(sizeof(double) * 3 * (size_t)ndihed));
-    SOFIA_CUDA(ctx, ctx->red_out.ensure(sizeof(double) * (16 + 8 * RED_BLOCKS)));
+    if ((rc = reduce_room(ctx))) return rc;
     SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->acc64.p, 0, sizeof(double) * 3 * (size_t)np, st));
     SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t) * sofia::ST_NSLOTS, st));
     DsfConst k = make_const(box, ibox, rcut2, cut_coulsq, alpha, e_shift, f_shift, coulpre);
-    k_dihedral_dsf<<<sofia::grid_for(ndihed, 128), 128, 0, st>>>(
+    sofia::launch_pdl(k_dihedral_dsf, sofia::grid_for(ndihed, 128), 128, 0, st,
         ndihed, np, (const float4 *)dpos, (const float *)dq, ntypes, (const double *)dlj,
         (const int *)ddl, (const double *)ddc, ndihedtypes, k, box, ibox,
         ctx->acc64.as<double>(), ctx->pe_atom.as<double>(), ctx->d_status);
-    reduce_cols(st, ndihed, 3, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 1.0);
-    k_add_to_float<<<sofia::grid_for(3L * np, 256), 256, 0, st>>>(3L * np, ctx->acc64.as<double>(),
+    reduce_cols<3>(st, ndihed, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 1.0);
+    sofia::launch_pdl(k_add_to_float, sofia::grid_for(3L * np, 256), 256, 0, st, 3L * np, ctx->acc64.as<double>(),
                                                                   (float *)o_ff.dev);
     SOFIA_CUDA(ctx, cudaGetLastError());
     if ((rc = sofia::finish_out(ctx, o_ff))) return rc;
@@ -1295,6 +1312,7 @@ __global__ void k_improper_ref(int nimpro, int np, const float4 *__restrict__ po
                                const int *__restrict__ il, const double *__restrict__ ic,
                                int nimprotypes, float box, float ibox, double *__restrict__ acc,
                                double *__restrict__ pe, int *__restrict__ status) {
+    SOFIA_PDL_ENTRY();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nimpro) return;
     const int i1 = il[5 * m] - 1, i2 = il[5 * m + 1] - 1, i3 = il[5 * m + 2] - 1,
@@ -1354,14 +1372,14 @@ extern "C" int sofia_improper_harmonic(sofia_nb_ctx *ctx, int np, const sofia_ai
         return rc;
     SOFIA_CUDA(ctx, ctx->acc64.ensure(sizeof(double) * 3 * (size_t)np));
     SOFIA_CUDA(ctx, ctx->pe_atom.ensure(sizeof(double) * 4 * (size_t)nimpro));
-    SOFIA_CUDA(ctx, ctx->red_out.ensure(sizeof(double) * (16 + 8 * RED_BLOCKS)));
+    if ((rc = reduce_room(ctx))) return rc;
     SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->acc64.p, 0, sizeof(double) * 3 * (size_t)np, st));
     SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t) * sofia::ST_NSLOTS, st));
-    k_improper_ref<<<sofia::grid_for(nimpro, 128), 128, 0, st>>>(
+    sofia::launch_pdl(k_improper_ref, sofia::grid_for(nimpro, 128), 128, 0, st,
         nimpro, np, (const float4 *)dpos, (const int *)dil, (const double *)dic, nimprotypes, box,
         ibox, ctx->acc64.as<double>(), ctx->pe_atom.as<double>(), ctx->d_status);
-    reduce_cols(st, nimpro, 4, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 1.0);
-    k_add_to_float<<<sofia::grid_for(3L * np, 256), 256, 0, st>>>(3L * np, ctx->acc64.as<double>(),
+    reduce_cols<4>(st, nimpro, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 1.0);
+    sofia::launch_pdl(k_add_to_float, sofia::grid_for(3L * np, 256), 256, 0, st, 3L * np, ctx->acc64.as<double>(),
                                                                   (float *)o_ff.dev);
     SOFIA_CUDA(ctx, cudaGetLastError());
     if ((rc = sofia::finish_out(ctx, o_ff))) return rc;
@@ -1611,16 +1629,16 @@ extern "C" int sofia_correct_1x(sofia_nb_ctx *ctx, int np, const sofia_ainfo *po
     if ((rc = sofia::stage_out(ctx, ffc, sizeof(float) * 3 * (size_t)np, 3, &o_ff, true))) return rc;
     SOFIA_CUDA(ctx, ctx->acc64.ensure(sizeof(double) * 3 * (size_t)np));
     SOFIA_CUDA(ctx, ctx->pe_atom.ensure(sizeof(double) * 4 * (size_t)npairs));
-    SOFIA_CUDA(ctx, ctx->red_out.ensure(sizeof(double) * (16 + 8 * RED_BLOCKS)));
+    if ((rc = reduce_room(ctx))) return rc;
     SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->acc64.p, 0, sizeof(double) * 3 * (size_t)np, st));
     DsfConst k = make_const(box, ibox, 0.0, cut_coulsq, 0.0, 0.0, 0.0, coulpre);
     SOFIA_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t) * sofia::ST_NSLOTS, st));
-    k_correct_pairs<<<sofia::grid_for(npairs, 128), 128, 0, st>>>(
+    sofia::launch_pdl(k_correct_pairs, sofia::grid_for(npairs, 128), 128, 0, st,
         npairs, np, (const float4 *)dpos, (const float *)dq, (const int *)dlist, stride, col_a,
         col_b, k, gewald, fudge, coulpre, ctx->acc64.as<double>(), ctx->pe_atom.as<double>(),
         ctx->d_status);
-    reduce_cols(st, npairs, 4, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 1.0);
-    k_add_to_float<<<sofia::grid_for(3L * np, 256), 256, 0, st>>>(3L * np, ctx->acc64.as<double>(),
+    reduce_cols<4>(st, npairs, ctx->pe_atom.as<double>(), ctx->red_out.as<double>(), 1.0);
+    sofia::launch_pdl(k_add_to_float, sofia::grid_for(3L * np, 256), 256, 0, st, 3L * np, ctx->acc64.as<double>(),
                                                                   (float *)o_ff.dev);
     SOFIA_CUDA(ctx, cudaGetLastError());
     if ((rc = sofia::finish_out(ctx, o_ff))) return rc;
@@ -1722,7 +1740,8 @@ extern "C" int sofia_force_nonbond_dsf_noalloc(
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     double *pe = scratch;
     double *out = scratch + (size_t)SOFIA_NOALLOC_MAX_ATOMS * 5;
-    // every scratch element this call reads is first written by this call
+    // every scratch element this call reads is first written by this call, but for the
+    // reduction's counter, which starts at zero with the image and ends every call there
     // (k_force_ref fills pe[0..5*np), the reduction fills its partials and out),
     // so nothing needs clearing between calls
     DsfConst k = make_const(box, ibox, rcut2, cut_coulsq, alpha, e_shift, f_shift, coulpre);
@@ -1730,7 +1749,7 @@ extern "C" int sofia_force_nonbond_dsf_noalloc(
     k_force_ref<<<sofia::grid_for(threads, 256), 256, 0, st>>>(
         np, (const float4 *)position, q, lj1, lj2, lj3, lj4, ntypes, nlist, numneigh, neigh_alloc,
         k, ff, pe);
-    reduce_cols(st, np, 5, pe, out, 0.5);
+    reduce_cols<5>(st, np, pe, out, 0.5);
     double h[5];
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
