@@ -70,8 +70,8 @@ __global__ void k_kick(int n, double h, const double *__restrict__ invm,
 // previous step's list decisions).  TWICE: the previous step's closing
 // half-kick first, as its own rounded addition (v += h f / m twice with the same
 // forces), so a segment that skips the separate closing kick gives the same bits.
-// CLEAR: the forces, just used up, are set to zero for the step's terms to add to.
-template <bool TWICE, bool CLEAR>
+// The forces, just used up, are set to zero for the step's terms to add to.
+template <bool TWICE>
 __device__ __forceinline__ void kick_drift_body(int bx, int n, double h, const double *__restrict__ invm,
                              long long *__restrict__ fx, long long *__restrict__ fy,
                              long long *__restrict__ fz, double *__restrict__ vx,
@@ -97,11 +97,9 @@ __device__ __forceinline__ void kick_drift_body(int bx, int n, double h, const d
         ux = ux + gx;
         uy = uy + gy;
         uz = uz + gz;
-        if (CLEAR) {
-            fx[i] = 0;
-            fy[i] = 0;
-            fz[i] = 0;
-        }
+        fx[i] = 0;
+        fy[i] = 0;
+        fz[i] = 0;
         vx[i] = ux;
         vy[i] = uy;
         vz[i] = uz;
@@ -127,7 +125,7 @@ __global__ void k_kick_drift(int n, double h, const double *__restrict__ invm,
                              const double *__restrict__ pz, double L, double lim2, double plim2,
                              int *__restrict__ flag, long long *__restrict__ step) {
     SOFIA_PDL_ENTRY();
-    kick_drift_body<TWICE, true>(blockIdx.x, n, h, invm, fx, fy, fz, vx, vy, vz, dt, x, y, z, rx, ry, rz, px, py, pz, L, lim2, plim2, flag, step);
+    kick_drift_body<TWICE>(blockIdx.x, n, h, invm, fx, fy, fz, vx, vy, vz, dt, x, y, z, rx, ry, rz, px, py, pz, L, lim2, plim2, flag, step);
 }
 
 
@@ -1376,7 +1374,7 @@ template <bool TWICE>
 __global__ void __launch_bounds__(256, SOFIA_BATCH_STREAM_MINB) k_kick_drift_b(BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_A256)
-    kick_drift_body<TWICE, false>(lb, d.n, d.h, d.invm, d.fx, d.fy, d.fz, d.vx, d.vy, d.vz, d.dt, d.x, d.y,
+    kick_drift_body<TWICE>(lb, d.n, d.h, d.invm, d.fx, d.fy, d.fz, d.vx, d.vy, d.vz, d.dt, d.x, d.y,
                     d.z, d.rx, d.ry, d.rz, d.px, d.py, d.pz, d.L, d.lim2, d.plim2, d.flag,
                     d.step);
     SOFIA_BATCH_END
@@ -1531,18 +1529,24 @@ static void repdev_fill_md(Sys *s, RepDev *d) {
 // One batched MD step: the same kernels, in the same order, as md_step.
 // One batch step; twice and close as for md_step (a segment chains its steps'
 // closing half-kicks into the next steps' kick and drift).
-static void batch_step(BatchDev *tab, Sys *s0, bool energy, bool rattle, cudaStream_t st,
+// The bonded terms run beside the list maintenance and the pair kernel, as in a step of
+// one system (md_forces): ctx's side stream and its events are open.
+static void batch_step(BatchDev *tab, Sys *s0, bool energy, bool rattle, sofia_nb_ctx *ctx,
                        int nsm, int pair_blocks, bool twice = false, bool close = true) {
     const int g256 = nsm * 8, g128 = nsm * 16;
+    cudaStream_t st = ctx->stream;
     if (twice)
         launch_pdl(k_kick_drift_b<true>, g256, 256, 0, st, tab);
     else
         launch_pdl(k_kick_drift_b<false>, g256, 256, 0, st, tab);
-    batch_pair_path(tab, s0, s0->precision, energy, st, nsm, pair_blocks);
+    cudaEventRecord(ctx->fork, st);
+    cudaStreamWaitEvent(ctx->side, ctx->fork, 0);
     if (energy)
-        launch_pdl(k_bonded_b<true>, g128, 128, 0, st, tab);
+        launch_pdl(k_bonded_b<true>, g128, 128, 0, ctx->side, tab);
     else
-        launch_pdl(k_bonded_b<false>, g128, 128, 0, st, tab);
+        launch_pdl(k_bonded_b<false>, g128, 128, 0, ctx->side, tab);
+    cudaEventRecord(ctx->join, ctx->side);
+    batch_pair_path(tab, s0, s0->precision, energy, st, nsm, pair_blocks, ctx->join);
     launch_pdl(k_shake_b, g128, 128, 0, st, tab);
     if (!close) return;
     launch_pdl(k_kick_b, g256, 256, 0, st, tab);
@@ -1695,6 +1699,7 @@ extern "C" int sofia_batch_set_segment(sofia_batch *b, int steps) {
 static int batch_capture(sofia_batch *b) {
     batch_drop_graphs(b);
     sofia_nb_ctx *ctx = b->ctx;
+    SOFIA_CUDA(ctx, sofia::side_open(ctx));
     cudaStream_t ms = ctx->stream;
     auto *tab = b->tab.as<sofia::BatchDev>();
     Sys *s0 = &b->sys[0]->s;
@@ -1710,7 +1715,7 @@ static int batch_capture(sofia_batch *b) {
         const bool fuse = !rat;
         for (int k = 0; k < nsteps[g]; ++k) {
             const bool last = k == nsteps[g] - 1;
-            sofia::batch_step(tab, s0, (g & 1) && last, rat, ms, b->nsm, pair_blocks,
+            sofia::batch_step(tab, s0, (g & 1) && last, rat, ctx, b->nsm, pair_blocks,
                               fuse && k > 0, !fuse || last);
         }
         cudaError_t ce = cudaStreamEndCapture(ms, &graph);

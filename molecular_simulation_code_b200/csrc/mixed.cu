@@ -2680,7 +2680,7 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4) ? (EN ? SOFIA_PAIR_MINB_
 __global__ void __launch_bounds__(256, SOFIA_BATCH_STREAM_MINB) k_unpack_b(const BatchDev *__restrict__ tab) {
     SOFIA_PDL_ENTRY();
     SOFIA_BATCH_LOOP(BK_S256)
-    unpack_body<false>(lb, d.nslots, d.ncl, d.slot_orig, reinterpret_cast<const long long *>(d.fslot),
+    unpack_body<true>(lb, d.nslots, d.ncl, d.slot_orig, reinterpret_cast<const long long *>(d.fslot),
                 d.fx, d.fy, d.fz, d.ctx_status, d.flag, d.dcount, d.lg, nullptr);
     SOFIA_BATCH_END
 }
@@ -2860,8 +2860,8 @@ cudaError_t batch_pair_smem_optin(int nt) {
 }
 
 void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
-                     cudaStream_t st, int nsm, int pair_blocks) {
-    const int g256 = nsm * 8, g128 = nsm * 16;
+                     cudaStream_t st, int nsm, int pair_blocks, cudaEvent_t join) {
+    const int g256 = nsm * 8;
     launch_pdl(k_batch_active_b, 1, MAXREP, 0, st, tab);
     launch_pdl(k_wrap_bin_b, g256, 256, 0, st, tab);
     launch_pdl(k_scan_cols_b, nsm * 2, 1024, 0, st, tab);
@@ -2889,7 +2889,9 @@ void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
         else
             launch_pdl(k_pair_b<float, false, false, true>, gw, 256, smem, st, tab, k);
     }
-    launch_pdl(k_unpack_b, g256, 256, 0, st, tab);
+    // two predecessors: a plain launch, which waits for both
+    cudaStreamWaitEvent(st, join, 0);
+    k_unpack_b<<<g256, 256, 0, st>>>(tab);
     if (energy) {
         launch_pdl(k_red_stage1_b, g256, 256, 0, st, tab);
         launch_pdl(k_red_stage2_b, nsm * 2, 256, 0, st, tab);

@@ -281,8 +281,9 @@ void repdev_fill_pair(const Sys *s, RepDev *d);
 // pair_blocks: the warp-per-cluster virtual blocks over all members when the graph
 // is captured, the grid of the pair, search and prune kernels (later members that
 // need more are covered by the kernels' grid-stride loops).
+// join: work that the force unpack waits for; it adds to the force arrays.
 void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
-                     cudaStream_t st, int nsm, int pair_blocks);
+                     cudaStream_t st, int nsm, int pair_blocks, cudaEvent_t join);
 // raises the batched pair kernels' dynamic shared-memory limit for nt atom types
 cudaError_t batch_pair_smem_optin(int nt);
 // The pair constants a captured batch graph holds (everything but the box).
