@@ -1532,7 +1532,8 @@ static void repdev_fill_md(Sys *s, RepDev *d) {
 // The bonded terms run beside the list maintenance and the pair kernel, as in a step of
 // one system (md_forces): ctx's side stream and its events are open.
 static void batch_step(BatchDev *tab, Sys *s0, bool energy, bool rattle, sofia_nb_ctx *ctx,
-                       int nsm, int pair_blocks, bool twice = false, bool close = true) {
+                       int nsm, int row_blocks, int pair_blocks, int split, bool twice = false,
+                       bool close = true) {
     const int g256 = nsm * 8, g128 = nsm * 16;
     cudaStream_t st = ctx->stream;
     if (twice)
@@ -1546,7 +1547,8 @@ static void batch_step(BatchDev *tab, Sys *s0, bool energy, bool rattle, sofia_n
     else
         launch_pdl(k_bonded_b<false>, g128, 128, 0, ctx->side, tab);
     cudaEventRecord(ctx->join, ctx->side);
-    batch_pair_path(tab, s0, s0->precision, energy, st, nsm, pair_blocks, ctx->join);
+    batch_pair_path(tab, s0, s0->precision, energy, st, nsm, row_blocks, pair_blocks, split,
+                    ctx->join);
     launch_pdl(k_shake_b, g128, 128, 0, st, tab);
     if (!close) return;
     launch_pdl(k_kick_b, g256, 256, 0, st, tab);
@@ -1570,6 +1572,7 @@ struct sofia_batch {
     std::vector<int> hstat;             // their host copies
     std::vector<double> hestat;
     int seg = 100;                      // steps per captured segment graph
+    int split = 1;                      // warps per list row of the force-only pair kernel
     int nsm = 148;
     // captured graphs: [0] one step, [1] one step with energies, [2] seg steps,
     // [3] seg steps with energies on the last
@@ -1617,6 +1620,11 @@ static int batch_upload(sofia_batch *b) {
     if (b->htab.size() != sizeof(sofia::BatchDev)) b->htab.assign(sizeof(sofia::BatchDev), 0);
     auto *h = reinterpret_cast<sofia::BatchDev *>(b->htab.data());
     h->nrep = n;
+    if (!b->graph_ok) {  // the captured graphs keep the split they were captured with
+        std::vector<const Sys *> members;
+        for (auto *m : b->sys) members.push_back(&m->s);
+        b->split = sofia::batch_pair_split(members);
+    }
     for (int k = 0; k < sofia::BK_N; ++k) h->pre[k][0] = 0;
     for (int r = 0; r < n; ++r) {
         Sys *s = &b->sys[r]->s;
@@ -1627,6 +1635,7 @@ static int batch_upload(sofia_batch *b) {
         const int cnt[sofia::BK_N] = {
             sofia::grid_for(s->n, 256), 1, s->ncols, sofia::grid_for((long)s->max_clusters * 8, 256),
             sofia::grid_for((long)s->max_clusters * 32, 256),
+            sofia::grid_for((long)s->max_clusters * 32 * b->split, 128),
             sofia::grid_for(nterm, 128), sofia::grid_for(s->md.nshake, 128), sofia::RED_BLOCKS,
             1, sofia::MD_NJOB * sofia::MRED, sofia::MD_NJOB};
         for (int k = 0; k < sofia::BK_N; ++k) h->pre[k][r + 1] = h->pre[k][r] + cnt[k];
@@ -1707,7 +1716,8 @@ static int batch_capture(sofia_batch *b) {
     for (auto *s : b->sys) rat = rat || (s->s.md.rattle && s->s.md.nshake);
     const int nsteps[4] = {1, 1, b->seg, b->seg};
     const auto *h = reinterpret_cast<const sofia::BatchDev *>(b->htab.data());
-    const int pair_blocks = h->pre[sofia::BK_W256][h->nrep];
+    const int row_blocks = h->pre[sofia::BK_W256][h->nrep];
+    const int pair_blocks = h->pre[sofia::BK_P128][h->nrep];
     for (int g = 0; g < 4; ++g) {
         cudaGraph_t graph = nullptr;
         SOFIA_CUDA(ctx, cudaStreamBeginCapture(ms, cudaStreamCaptureModeThreadLocal));
@@ -1715,7 +1725,8 @@ static int batch_capture(sofia_batch *b) {
         const bool fuse = !rat;
         for (int k = 0; k < nsteps[g]; ++k) {
             const bool last = k == nsteps[g] - 1;
-            sofia::batch_step(tab, s0, (g & 1) && last, rat, ctx, b->nsm, pair_blocks,
+            sofia::batch_step(tab, s0, (g & 1) && last, rat, ctx, b->nsm, row_blocks,
+                              pair_blocks, b->split,
                               fuse && k > 0, !fuse || last);
         }
         cudaError_t ce = cudaStreamEndCapture(ms, &graph);

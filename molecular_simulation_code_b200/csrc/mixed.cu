@@ -1929,12 +1929,11 @@ int sys_eval(Sys *s, int precision, bool energy, bool virial, bool force_build) 
 // 80, 37,000 125 / 123 / 134, 275,000 605 / 626 / 750).  FP64 runs half as many warps
 // and is bound by its pipe sooner: 2 only while both fit (3,000 atoms 116 / 89 / -,
 // 9,000 128 / 100 / 127, 16,000 140 / 143 / -).
-static int pair_split(const Sys *s, int precision) {
+static int pair_split(const Sys *s, int precision, long rows) {
     // the table of this many types allows one block less per SM: one warp per row
     if (pair_smem(s->ntypes, false, true) > 32768) return 1;
     const bool mixed = precision != SOFIA_PREC_FP64;
     const long res = (long)s->nsm * (mixed ? 32 : 16);  // resident warps
-    const long rows = expected_rows(s);
     if (4 * rows <= res) return 4;
     return (mixed ? rows : 2 * rows) <= res ? 2 : 1;
 }
@@ -1982,7 +1981,7 @@ int sys_pair(Sys *s, int precision, bool energy, bool virial, int *count_flag,
     sofia_nb_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     PairConst k = make_pair_const(s, nullptr);
-    const int split = pair_split(s, precision);
+    const int split = pair_split(s, precision, expected_rows(s));
     if (s->timing) cudaEventRecord(s->ev[2], st);
     // sofia_system_create requires rcut == cut_coul: one cut-off gates both terms
     if (split == 4)
@@ -2666,13 +2665,21 @@ __global__ void __launch_bounds__(256, SOFIA_PRUNE_MINB) k_prune_b(BatchDev *__r
     SOFIA_BATCH_END
 }
 
-template <typename T, bool EN, bool VIR, bool SAME, bool TRI = false>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4) ? (EN ? SOFIA_PAIR_MINB_EN : SOFIA_PAIR_MINB) : 2)
+// Energy steps take blocks of 256 threads with one warp per row, the other steps blocks
+// of 128 with SPLIT warps per row, as a single system does: a batch whose rows leave
+// warps idle shares them (2 replicas of 12,841 atoms 121 -> 97 us per step; 4 of 51,001
+// and 16 of 174,085 keep one warp per row, 190 and 493 us).
+template <bool EN>
+constexpr int batch_pair_block() { return EN ? 256 : 128; }
+template <typename T, bool EN, bool SAME, bool TRI = false, int SPLIT = 1>
+__global__ void __launch_bounds__(batch_pair_block<EN>(),
+                                  (sizeof(T) == 4 ? (EN ? SOFIA_PAIR_MINB_EN : SOFIA_PAIR_MINB) : 2) *
+                                      256 / batch_pair_block<EN>())
     k_pair_b(BatchDev *__restrict__ tab, PairConst k) {
     SOFIA_PDL_ENTRY();
-    SOFIA_BATCH_LOOP(BK_W256)
-    pair_body<T, EN, VIR, SAME, TRI, 1>(lb, d.maxcl, d.ncl, d.rec, d.ilist, d.imask, d.icount, d.jcap,
-                                d.ljtab, k, d.L, d.fslot, d.energy);
+    SOFIA_BATCH_LOOP(EN ? BK_W256 : BK_P128)
+    pair_body<T, EN, false, SAME, TRI, SPLIT>(lb, d.maxcl, d.ncl, d.rec, d.ilist, d.imask, d.icount,
+                                              d.jcap, d.ljtab, k, d.L, d.fslot, d.energy);
     __syncthreads();
     SOFIA_BATCH_END
 }
@@ -2851,16 +2858,22 @@ cudaError_t batch_pair_smem_optin(int nt) {
         const cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
         if (r != cudaSuccess) e = r;
     };
-    set((const void *)k_pair_b<double, true, false, true>);
-    set((const void *)k_pair_b<double, false, false, true>);
-    set((const void *)k_pair_b<float, true, false, true>);
-    set((const void *)k_pair_b<float, false, false, true>);
+    set((const void *)k_pair_b<double, true, true>);
+    set((const void *)k_pair_b<double, false, true>);
+    set((const void *)k_pair_b<float, true, true>);
+    set((const void *)k_pair_b<float, false, true>);
     if (e == cudaSuccess) done = need;
     return e;
 }
 
+int batch_pair_split(const std::vector<const Sys *> &members) {
+    long rows = 0;
+    for (const Sys *s : members) rows += expected_rows(s);
+    return pair_split(members[0], members[0]->precision, rows);
+}
+
 void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
-                     cudaStream_t st, int nsm, int pair_blocks, cudaEvent_t join) {
+                     cudaStream_t st, int nsm, int row_blocks, int pair_blocks, int split, cudaEvent_t join) {
     const int g256 = nsm * 8;
     launch_pdl(k_batch_active_b, 1, MAXREP, 0, st, tab);
     launch_pdl(k_wrap_bin_b, g256, 256, 0, st, tab);
@@ -2869,25 +2882,32 @@ void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
     launch_pdl(k_pack_b, g256, 256, 0, st, tab);
     // one block per warp-per-cluster virtual block of all members (blocks past the
     // replicas whose trigger fired return at once)
-    const int gw = pair_blocks > 0 ? pair_blocks : 1;
+    const int gw = row_blocks > 0 ? row_blocks : 1;
     launch_pdl(k_search_b, gw, 256, 0, st, tab);
     launch_pdl(k_prune_b, gw, 256, 0, st, tab);
     const PairConst k = make_pair_const(s0, nullptr);
     const size_t smem = pair_smem(s0->ntypes, false, energy);
-    const bool tri = energy && pair_tri(s0->ntypes);
-    const size_t smem3 = pair_smem(s0->ntypes, tri, energy);
-    if (precision == SOFIA_PREC_FP64) {
-        if (energy)
-            launch_pdl(k_pair_b<double, true, false, true>, gw, 256, smem, st, tab, k);
+    const bool fp64 = precision == SOFIA_PREC_FP64;
+    if (energy) {
+        const bool tri = pair_tri(s0->ntypes);
+        const size_t smem3 = pair_smem(s0->ntypes, tri, true);
+        if (fp64)
+            launch_pdl(k_pair_b<double, true, true>, gw, 256, smem, st, tab, k);
+        else if (tri)
+            launch_pdl(k_pair_b<float, true, true, true>, gw, 256, smem3, st, tab, k);
         else
-            launch_pdl(k_pair_b<double, false, false, true>, gw, 256, smem, st, tab, k);
-    } else if (tri) {
-        launch_pdl(k_pair_b<float, true, false, true, true>, gw, 256, smem3, st, tab, k);
+            launch_pdl(k_pair_b<float, true, true>, gw, 256, smem, st, tab, k);
     } else {
-        if (energy)
-            launch_pdl(k_pair_b<float, true, false, true>, gw, 256, smem, st, tab, k);
+        const int gp = pair_blocks > 0 ? pair_blocks : 1;
+        auto go = [&](auto kernel) { launch_pdl(kernel, gp, 128, smem, st, tab, k); };
+        if (fp64)
+            split == 4 ? go(k_pair_b<double, false, true, false, 4>)
+                       : split == 2 ? go(k_pair_b<double, false, true, false, 2>)
+                                    : go(k_pair_b<double, false, true>);
         else
-            launch_pdl(k_pair_b<float, false, false, true>, gw, 256, smem, st, tab, k);
+            split == 4 ? go(k_pair_b<float, false, true, false, 4>)
+                       : split == 2 ? go(k_pair_b<float, false, true, false, 2>)
+                                    : go(k_pair_b<float, false, true>);
     }
     // two predecessors: a plain launch, which waits for both
     cudaStreamWaitEvent(st, join, 0);

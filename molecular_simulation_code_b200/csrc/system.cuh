@@ -15,6 +15,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <vector>
+
 #include "common.cuh"
 #include "langevin.cuh"
 
@@ -168,6 +170,7 @@ enum BatchKind {
     BK_COLS,      // ncols: the column sort
     BK_S256,      // ceil(max_clusters * 8 / 256): per-slot kernels
     BK_W256,      // ceil(max_clusters * 32 / 256): warp-per-cluster kernels
+    BK_P128,      // ceil(max_clusters * 32 * split / 128): the force-only pair kernel
     BK_B128,      // ceil(bonded terms / 128)
     BK_G128,      // ceil(SHAKE groups / 128)
     BK_RED,       // RED_BLOCKS: stage 1 of the pair-energy sums
@@ -278,12 +281,17 @@ void repdev_fill_pair(const Sys *s, RepDev *d);
 // Langevin force, and (energy) the pair-energy sums.  All replicas share the
 // pair constants k (all but the box) and the precision.
 // nsm: multiprocessors of the device (the grid-stride launches are sized from it).
-// pair_blocks: the warp-per-cluster virtual blocks over all members when the graph
-// is captured, the grid of the pair, search and prune kernels (later members that
-// need more are covered by the kernels' grid-stride loops).
+// row_blocks, pair_blocks: the BK_W256 and BK_P128 virtual blocks over all members when
+// the graph is captured, the grids of the energy pair, search and prune kernels and of
+// the force-only pair kernel (later members that need more are covered by the kernels'
+// grid-stride loops); split: warps per list row of the latter, for which the table's
+// BK_P128 prefixes are made.
 // join: work that the force unpack waits for; it adds to the force arrays.
 void batch_pair_path(BatchDev *tab, const Sys *s0, int precision, bool energy,
-                     cudaStream_t st, int nsm, int pair_blocks, cudaEvent_t join);
+                     cudaStream_t st, int nsm, int row_blocks, int pair_blocks, int split,
+                     cudaEvent_t join);
+// Warps per list row of the force-only pair kernel for these members.
+int batch_pair_split(const std::vector<const Sys *> &members);
 // raises the batched pair kernels' dynamic shared-memory limit for nt atom types
 cudaError_t batch_pair_smem_optin(int nt);
 // The pair constants a captured batch graph holds (everything but the box).
