@@ -62,11 +62,9 @@ __global__ void k_bin_atoms(int np, const float4 *__restrict__ pos, double boxd,
     if (!(inside(p.x) && inside(p.y) && inside(p.z))) status[sofia::ST_UNWRAPPED] = 1;
 }
 
-constexpr int LIST_ATOMS = 8;  // atoms per warp of the list build
-
 // Exclusive scans by one block (cells are few): of the n cell counts into
-// start[0..n], and of the cells' chunks of LIST_ATOMS atoms into chunk[0..n].
-__global__ void __launch_bounds__(1024) k_scan_block(int n, const int *__restrict__ in,
+// start[0..n], and of the cells' chunks of `atoms` atoms into chunk[0..n].
+__global__ void __launch_bounds__(1024) k_scan_block(int n, int atoms, const int *__restrict__ in,
                                                      int *__restrict__ start,
                                                      int *__restrict__ chunk) {
     SOFIA_PDL_ENTRY();
@@ -74,7 +72,7 @@ __global__ void __launch_bounds__(1024) k_scan_block(int n, const int *__restric
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     int2 carry = make_int2(0, 0);
     for (int base = 0; base < n; base += 1024) {
-        const int v = (base + t < n) ? in[base + t] : 0, u = (v + LIST_ATOMS - 1) / LIST_ATOMS;
+        const int v = (base + t < n) ? in[base + t] : 0, u = (v + atoms - 1) / atoms;
         int2 incl = make_int2(v, u);
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
@@ -189,11 +187,11 @@ __global__ void __launch_bounds__(256) k_sort_cells(
 
 // build_neighbor_nonewton_nomic, mod_neighbor.f90:622-809, over the stencil of
 // neighcell_nonewton (:1309-1378): the own cell, then the 26 others z-major.
-// A warp takes a chunk of 8 atoms of one cell and sweeps the stencil's atoms in
-// order, 32 candidates at a time: they are staged in shared memory, lane (a, q) tests
-// atom a against candidates 8q .. 8q + 7, two per packed FP32x2 operation, and keeps
-// the outcomes as sign bits; the four lanes of an atom combine them to its 32-bit
-// mask, and the warp writes each atom's survivors compacted by that mask, coalesced
+// A warp takes a chunk of ATOMS (4 or 8) atoms of one cell and sweeps the stencil's
+// atoms in order, 32 candidates at a time: they are staged in shared memory, lane
+// (a, q) tests atom a against candidates ATOMS q .. ATOMS q + ATOMS - 1, two per packed
+// FP32x2 operation, and keeps the outcomes as sign bits; the lanes of an atom combine
+// them to its 32-bit mask, and the warp writes each atom's survivors compacted by that mask, coalesced
 // and in the reference's order.
 //
 // The sweep is bound by instruction issue (about 3,600 candidates per atom at 10.9 A
@@ -209,7 +207,7 @@ __global__ void __launch_bounds__(256) k_sort_cells(
 //     that is the sign of dr2 - lim;
 //   * an atom and its partners become a mask over the 32 candidates, made only for
 //     tiles that can hold one of them.
-// 45,255 atoms, 12 A: 224 us (171 M warp instructions); 527 us as one warp per atom
+// 45,255 atoms, 12 A: 234 us (182 M warp instructions); 527 us as one warp per atom
 // with the minimum image and 12 partner compares per candidate, 254 us as one warp per
 // two atoms with a ballot per atom and 32 candidates, 227 us as one atom per lane with
 // a buffer column each (99 M instructions, but 12 warps per SM).
@@ -218,16 +216,21 @@ struct ListTile {
     float x[32], y[32], z[32];  // negated coordinates
 };
 
-// Sign bits of dr2 - lim for 8 candidates from place k0 on: bit k of the result is set
+// d - rint(d * ibox) * box for |d| <= box.
+__device__ __forceinline__ float list_image(float d, float box, float half) {
+    return fabsf(d) > half ? d - copysignf(box, d) : d;
+}
+
+// Sign bits of dr2 - lim for N candidates from place k0 on: bit k of the result is set
 // when candidate k0 + k survives.  IMG: 0 no image, 1 the run's image shift, 2 minimum
-// image per pair.
-template <int IMG>
+// image per pair, 3 the same for coordinates in [0, box].
+template <int IMG, int N>
 __device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 px, float2 py,
                                               float2 pz, float3 sh, float box, float ibox,
-                                              float nlim) {
+                                              float half, float nlim) {
     unsigned acc = 0u;
 #pragma unroll
-    for (int k = 4; k >= 0; k -= 4) {
+    for (int k = N - 4; k >= 0; k -= 4) {
         const float4 cx = *reinterpret_cast<const float4 *>(t.x + k0 + k),
                      cy = *reinterpret_cast<const float4 *>(t.y + k0 + k),
                      cz = *reinterpret_cast<const float4 *>(t.z + k0 + k);
@@ -240,6 +243,10 @@ __device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 
                 dx = __fadd2_rn(dx, make_float2(sh.x, sh.x));
                 dy = __fadd2_rn(dy, make_float2(sh.y, sh.y));
                 dz = __fadd2_rn(dz, make_float2(sh.z, sh.z));
+            } else if (IMG == 3) {
+                dx = make_float2(list_image(dx.x, box, half), list_image(dx.y, box, half));
+                dy = make_float2(list_image(dy.x, box, half), list_image(dy.y, box, half));
+                dz = make_float2(list_image(dz.x, box, half), list_image(dz.y, box, half));
             } else if (IMG == 2) {
                 // (b + sign(2^23,b)) - sign(2^23,dx) of :694-697 is rint(b) for |b| < 2^22
                 dx = make_float2(dx.x - rintf(dx.x * ibox) * box, dx.y - rintf(dx.y * ibox) * box);
@@ -252,7 +259,7 @@ __device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 
             const float r0 = __fadd_rn(__fadd_rn(xx.x, yy.x), zz.x),
                         r1 = __fadd_rn(__fadd_rn(xx.y, yy.y), zz.y);
             float2 d = make_float2(__fadd_rn(r0, nlim), __fadd_rn(r1, nlim));
-            if (IMG == 2) {  // a coordinate that is not finite survives nowhere
+            if (IMG >= 2) {  // a coordinate that is not finite survives nowhere
                 d.x = r0 < -nlim ? -1.0f : 1.0f;
                 d.y = r1 < -nlim ? -1.0f : 1.0f;
             }
@@ -263,11 +270,12 @@ __device__ __forceinline__ unsigned list_tile(const ListTile &t, int k0, float2 
     return acc;
 }
 
+template <int ATOMS>
 __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
     int np, int ncell, int D, const float4 *__restrict__ pair, const int *__restrict__ slot_of,
     const int *__restrict__ start, const int *__restrict__ chunk,
     const int *__restrict__ specbond, const int *__restrict__ num3bond, float box, float ibox,
-    float lim, int *__restrict__ nlist, int *__restrict__ numneigh, int neigh_alloc,
+    float half, float lim, int *__restrict__ nlist, int *__restrict__ numneigh, int neigh_alloc,
     int *__restrict__ status) {
     SOFIA_PDL_ENTRY();
     __shared__ __align__(16) ListTile s_tile[LIST_WARPS];
@@ -275,7 +283,7 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int job = blockIdx.x * LIST_WARPS + w;
     if (job >= chunk[ncell] || status[sofia::ST_CELLOVER]) return;  // an unsorted cell fails the call
-    const bool shift = D >= 5 && !status[sofia::ST_UNWRAPPED];
+    const bool inside = !status[sofia::ST_UNWRAPPED], shift = D >= 5 && inside;
     // the chunk's cell: the last one whose first chunk is not past this one
     int bin = 0;
     for (int lo = 0, hi = ncell - 1; lo <= hi;) {
@@ -317,13 +325,16 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
         s_seg[w][2][at] = code;
     }
     const int nseg = __popc(heads);
-    // atom a of the chunk; its lanes share the places of the atom (q = 3, last mark) and
-    // of its up to 12 partners (partner 4l + q is mark l of lane q)
-    const int a = lane & 7, q = lane >> 3;
-    const int s = start[bin] + LIST_ATOMS * (job - chunk[bin]) + a;
+    // atom a of the chunk; its lanes share the places of its up to 12 partners (partner
+    // LANES l + q is mark l of lane q) and of itself (q = 0, last mark)
+    constexpr int LANES = 32 / ATOMS, NPART = (12 + LANES - 1) / LANES;
+    const int a = lane % ATOMS, q = lane / ATOMS;
+    const int s = start[bin] + ATOMS * (job - chunk[bin]) + a;
     const bool live = s < start[bin + 1];
     float2 px = make_float2(0.0f, 0.0f), py = px, pz = px;
-    int id = 0, mark[4] = {-1, -1, -1, -1}, first = INT_MAX, last = -1;
+    int id = 0, mark[NPART + 1], first = INT_MAX, last = -1;
+#pragma unroll
+    for (int l = 0; l <= NPART; ++l) mark[l] = -1;
     if (live) {
         const float4 p = pair[s];
         px = make_float2(-p.x, -p.x);
@@ -332,14 +343,14 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
         id = __float_as_int(p.w);
         const int n3 = min(num3bond[id], 12);
 #pragma unroll
-        for (int l = 0; l < 3; ++l) {
-            if (4 * l + q >= n3) continue;
-            const int b = specbond[id * 12 + 4 * l + q];
+        for (int l = 0; l < NPART; ++l) {
+            if (LANES * l + q >= n3) continue;
+            const int b = specbond[id * 12 + LANES * l + q];
             if (b >= 1 && b <= np) mark[l] = slot_of[b - 1];  // others exclude nothing
         }
-        if (q == 3) mark[3] = s;
+        if (q == 0) mark[NPART] = s;
 #pragma unroll
-        for (int l = 0; l < 4; ++l)
+        for (int l = 0; l <= NPART; ++l)
             if (mark[l] >= 0) {
                 first = min(first, mark[l]);
                 last = max(last, mark[l]);
@@ -348,10 +359,10 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
     const int mfirst = __reduce_min_sync(FULL, first), mlast = __reduce_max_sync(FULL, last);
     const float nlim = live ? -lim : 1.0f;  // without an atom nothing survives (dr2 < -1)
     const unsigned below = (1u << lane) - 1u, bit = 1u << lane;
-    int *row[LIST_ATOMS];
-    int count[LIST_ATOMS];
+    int *row[ATOMS];
+    int count[ATOMS];
 #pragma unroll
-    for (int k = 0; k < LIST_ATOMS; ++k) {
+    for (int k = 0; k < ATOMS; ++k) {
         row[k] = nlist + (size_t)__shfl_sync(FULL, id, k) * (size_t)neigh_alloc;
         count[k] = 0;
     }
@@ -375,27 +386,33 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
             tile.y[lane] = p.y;
             tile.z[lane] = p.z;
             __syncwarp();
-#define SOFIA_TILE_ARGS tile, 8 * q, px, py, pz, sh, box, ibox, nlim
-            unsigned m = !shift ? list_tile<2>(SOFIA_TILE_ARGS)
-                       : cd != 21 ? list_tile<1>(SOFIA_TILE_ARGS) : list_tile<0>(SOFIA_TILE_ARGS);
+#define SOFIA_TILE_ARGS tile, ATOMS * q, px, py, pz, sh, box, ibox, half, nlim
+            unsigned m;
+            if (shift)
+                m = cd != 21 ? list_tile<1, ATOMS>(SOFIA_TILE_ARGS)
+                             : list_tile<0, ATOMS>(SOFIA_TILE_ARGS);
+            else if (ATOMS == 4 && inside)
+                m = list_tile<3, ATOMS>(SOFIA_TILE_ARGS);
+            else
+                m = list_tile<2, ATOMS>(SOFIA_TILE_ARGS);
 #undef SOFIA_TILE_ARGS
-            m <<= 8 * q;
-            m |= __shfl_xor_sync(FULL, m, 8);
-            m |= __shfl_xor_sync(FULL, m, 16);
+            m <<= ATOMS * q;
+#pragma unroll
+            for (int off = ATOMS; off < 32; off <<= 1) m |= __shfl_xor_sync(FULL, m, off);
             if (base <= mlast && base + 32 > mfirst) {
                 unsigned skip = 0u;
 #pragma unroll
-                for (int l = 0; l < 4; ++l) {
+                for (int l = 0; l <= NPART; ++l) {
                     const unsigned d = (unsigned)(mark[l] - base);
                     if (d < 32u) skip |= 1u << d;
                 }
-                skip |= __shfl_xor_sync(FULL, skip, 8);
-                skip |= __shfl_xor_sync(FULL, skip, 16);
+#pragma unroll
+                for (int off = ATOMS; off < 32; off <<= 1) skip |= __shfl_xor_sync(FULL, skip, off);
                 m &= ~skip;
             }
             const int cand = __float_as_int(p.w) + 1;
 #pragma unroll
-            for (int k = 0; k < LIST_ATOMS; ++k) {
+            for (int k = 0; k < ATOMS; ++k) {
                 const unsigned mk = __shfl_sync(FULL, m, k);
                 const int at = count[k] + __popc(mk & below);
                 if ((mk & bit) && at < neigh_alloc) row[k][at] = cand;
@@ -405,7 +422,7 @@ __global__ void __launch_bounds__(32 * LIST_WARPS) k_build_ref_list(
     }
     int most = 0;
 #pragma unroll
-    for (int k = 0; k < LIST_ATOMS; ++k) {
+    for (int k = 0; k < ATOMS; ++k) {
         if (lane == k && live) numneigh[id] = count[k];
         most = max(most, count[k]);
     }
@@ -972,6 +989,12 @@ int check_status(sofia_nb_ctx *ctx) {
     return ctx->copies->sync();
 }
 
+// Atoms per warp of the list build: a chunk's sweep over 3,600 candidates is one serial
+// chain, so a system whose chunks of 8 leave warps idle takes chunks of 4 (list plus FP64
+// forces at 3,300 / 9,000 / 15,900 atoms: 199 / 247 / 274 us with 8, 165 / 226 / 297 us
+// with 4).
+int list_atoms(int np) { return np < 12000 ? 4 : 8; }
+
 // Bin + sort shared by sofia_cell_sort and sofia_neighbor_build.  list: the sorted
 // positions go to pos_pair in the list build's form, with slot_of, instead of to
 // pos_sorted.
@@ -1002,7 +1025,8 @@ int cell_prepare(sofia_nb_ctx *ctx, int np, const float4 *dpos, float box, float
                       ctx->d_status);
     sofia::launch_pdl(k_bin_atoms, sofia::grid_for(np, 256), 256, 0, st, np, dpos, (double)box,
                       irn, nd, cell_of, rank, count, ctx->d_status);
-    sofia::launch_pdl(k_scan_block, 1, 1024, 0, st, nt, count, start, start + nt + 1);
+    sofia::launch_pdl(k_scan_block, 1, 1024, 0, st, nt, list_atoms(np), count, start,
+                      start + nt + 1);
     sofia::launch_pdl(k_scatter, sofia::grid_for(np, 256), 256, 0, st, np, cell_of, start, rank,
                       sorted);
     sofia::launch_pdl(k_sort_cells, nt, 256, 0, st, nt, start, sorted, descending, dpos,
@@ -1113,12 +1137,18 @@ extern "C" int sofia_neighbor_build(sofia_nb_ctx *ctx, int np, const sofia_ainfo
     float lim = (float)rv2;
     if ((double)lim < rv2) lim = nextafterf(lim, INFINITY);
     const int *start = ctx->cell_start.as<int>();
+    // rint(d * ibox) = 0 up to here, +-1 beyond
+    const float ibox = (float)(1.0 / (double)box);
+    float half = 0.5f * box;
+    while (half * ibox > 0.5f) half = nextafterf(half, 0.0f);
+    while (nextafterf(half, box) * ibox <= 0.5f) half = nextafterf(half, box);
     // at most one partial chunk per cell
-    sofia::launch_pdl(k_build_ref_list, sofia::grid_for((long)np / LIST_ATOMS + nt, LIST_WARPS),
-                      32 * LIST_WARPS, 0, st, np, nt, nd, ctx->pos_pair.as<float4>(),
-                      ctx->slot_of.as<int>(), start, start + nt + 1, (const int *)dsb,
-                      (const int *)dn3, box, (float)(1.0 / (double)box), lim, dlist, dnum,
-                      neigh_alloc, ctx->d_status);
+    const int atoms = list_atoms(np);
+    sofia::launch_pdl(atoms == 4 ? k_build_ref_list<4> : k_build_ref_list<8>,
+                      sofia::grid_for((long)np / atoms + nt, LIST_WARPS), 32 * LIST_WARPS, 0, st,
+                      np, nt, nd, ctx->pos_pair.as<float4>(), ctx->slot_of.as<int>(), start,
+                      start + nt + 1, (const int *)dsb, (const int *)dn3, box, ibox, half, lim,
+                      dlist, dnum, neigh_alloc, ctx->d_status);
     SOFIA_CUDA(ctx, cudaGetLastError());
     if ((rc = check_status(ctx))) return rc;
     if (ctx->h_status[sofia::ST_CELLOVER])
