@@ -1820,16 +1820,17 @@ extern "C" int sofia_batch_md_run(sofia_batch *b, int nsteps, int energy_every,
                                             cudaMemcpyDeviceToHost, ms));
         SOFIA_CUDA(ctx, cudaStreamSynchronize(ms));
         bool regrow = false;
+        int bad = SOFIA_OK;
         for (int i = 0; i < n; ++i) {
             Sys *s = &b->sys[i]->s;
             s->launches += launched / (n > 0 ? n : 1);
             const int r2 = sofia::sys_list_overflow(s, &b->hstat[(size_t)sofia::ST_NSLOTS * i]);
-            if (r2 == SOFIA_ENEEDGROW) {
+            if (r2 == SOFIA_ENEEDGROW)
                 regrow = true;
-                continue;
-            }
-            if (r2) return r2;
+            else if (r2 && !bad)
+                bad = r2;  // every member's words are looked at before the call fails
         }
+        if (bad) return bad;
         if (regrow) {
             // a list row overflowed: every replica restarts the segment from its
             // snapshot (the table is rewritten with the grown lists)

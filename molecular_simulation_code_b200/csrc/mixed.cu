@@ -1866,6 +1866,14 @@ static void sys_prune(Sys *s, const int *cond) {
 }
 
 
+// A build whose column overflowed has left atoms out: there is no list, and no
+// forces, until a later build succeeds.
+static int column_overflow(Sys *s) {
+    s->built = 0;
+    s->md.forces_valid = 0;
+    return fail(s->ctx, SOFIA_EINVAL, "an xy column holds more than 2048 atoms%s");
+}
+
 // One evaluation: displacement triggers, list rebuild or prune when due, pack,
 // pair kernel on the pruned list, deterministic energy reduction.
 int sys_eval(Sys *s, int precision, bool energy, bool virial, bool force_build) {
@@ -1906,8 +1914,7 @@ int sys_eval(Sys *s, int precision, bool energy, bool virial, bool force_build) 
             SOFIA_CUDA(ctx, cudaMemcpyAsync(hs, s->status_local.p, sizeof(hs),
                                             cudaMemcpyDeviceToHost, st));
             SOFIA_CUDA(ctx, cudaStreamSynchronize(st));
-            if (hs[ST_CELLOVER])
-                return fail(ctx, SOFIA_EINVAL, "an xy column holds more than 2048 atoms%s");
+            if (hs[ST_CELLOVER]) return column_overflow(s);
             if (hs[ST_NCLUSTER] > s->jcap) {
                 // redo with a larger row capacity, like the reference's list regrow
                 s->jcap = (int)(hs[ST_NCLUSTER] * 1.2) + 16;
@@ -2069,13 +2076,14 @@ int sys_list_overflow(Sys *s, const int32_t *status) {
                                         cudaMemcpyDeviceToHost, ctx->stream));
         SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
-    if (hs[ST_CELLOVER]) return fail(ctx, SOFIA_EINVAL, "an xy column holds more than 2048 atoms%s");
+    if (hs[ST_CELLOVER]) return column_overflow(s);
     if (hs[ST_NCLUSTER] > s->jcap) {
         s->jcap = (int)(hs[ST_NCLUSTER] * 1.2) + 16;
         int r2 = sys_alloc_list(s);
         if (r2) return r2;
         SOFIA_CUDA(ctx, cudaMemsetAsync(s->status_local.p, 0, sizeof(int) * ST_NSLOTS, ctx->stream));
         s->built = 0;
+        s->md.forces_valid = 0;  // made with truncated rows
         return SOFIA_ENEEDGROW;
     }
     return SOFIA_OK;
