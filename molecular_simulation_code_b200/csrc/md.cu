@@ -1018,7 +1018,7 @@ static int md_step(Sys *s, bool energy, bool twice = false, bool close = true) {
     return SOFIA_OK;
 }
 
-static void md_drop_graphs(Sys *s) {
+void md_drop_graphs(Sys *s) {
     for (auto &g : s->md.graph)
         if (g) {
             cudaGraphExecDestroy(g);

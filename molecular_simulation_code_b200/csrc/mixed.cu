@@ -1672,7 +1672,9 @@ void dropin_drop(Sys *s) {
 }
 
 static int sys_alloc_list(Sys *s) {
-    dropin_drop(s);  // captured drop-in graphs hold the old list pointers
+    // captured drop-in calls and MD steps hold the old list pointers
+    dropin_drop(s);
+    md_drop_graphs(s);
     const size_t maxcl = (size_t)s->max_clusters;
     SOFIA_CUDA(s->ctx, s->jlist.ensure(sizeof(int) * maxcl * s->jcap));
     SOFIA_CUDA(s->ctx, s->jmask.ensure(sizeof(unsigned long long) * maxcl * s->jcap));

@@ -338,6 +338,8 @@ int sys_list_overflow(Sys *s, const int32_t *status = nullptr);
 int forces_out(Sys *s, double *f);
 // Frees the captured drop-in force graphs (they bake in list pointers and the margin).
 void dropin_drop(Sys *s);
+// Frees the captured MD steps (they bake in the same).
+void md_drop_graphs(Sys *s);
 // Column grid and list capacities for a cluster shape (mixed.cu).
 bool sys_geometry(Sys *s, double aspect);
 // After a change of list geometry or margin (md.cu): drops the system's captured
