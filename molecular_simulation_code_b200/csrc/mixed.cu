@@ -2372,11 +2372,20 @@ extern "C" int sofia_system_set_state(sofia_system *ss, const double *x, const d
     sofia::DevBuf *dst[2] = {s->x, s->v};
     for (int k = 0; k < 2; ++k) {
         if (!src[k]) continue;
-        // a device array may still be written by work queued on the default stream
-        if (sofia::is_device_ptr(src[k])) SOFIA_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+        const size_t bytes = sizeof(double) * 3 * (size_t)s->n;
         const void *in;
-        const int rc = sofia::stage_in(ctx, src[k], sizeof(double) * 3 * (size_t)s->n, k, &in);
-        if (rc) return rc;
+        if (sofia::is_device_ptr(src[k])) {
+            // A copy, as the array may be on another GPU, made on the default stream, as
+            // work queued there or on a stream that waits for it may still write the array.
+            SOFIA_CUDA(ctx, ctx->stage[k].ensure(bytes));
+            in = ctx->stage[k].p;
+            SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            SOFIA_CUDA(ctx, cudaMemcpyAsync(ctx->stage[k].p, src[k], bytes, cudaMemcpyDefault,
+                                            cudaStreamLegacy));
+            SOFIA_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+        } else if (const int rc = sofia::stage_in(ctx, src[k], bytes, k, &in)) {
+            return rc;
+        }
         sofia::launch_pdl(sofia::k_state_in, sofia::grid_for(3L * s->n, 256), 256, 0, ctx->stream,
                           s->n, (const double *)in, dst[k][0].as<double>(),
                           dst[k][1].as<double>(), dst[k][2].as<double>());
@@ -2389,16 +2398,20 @@ extern "C" int sofia_system_set_state(sofia_system *ss, const double *x, const d
 
 namespace sofia {
 // The three components in atom order into the caller's [n][3] array (host or
-// device), delivered by the time of the call's sync(); stage: a staging slot.
+// device, this one or another), delivered by the time of the call's sync(); stage: a
+// staging slot.
 template <typename T>
 int state_out(Sys *s, const DevBuf (&v)[3], double *to, int stage) {
     sofia_nb_ctx *ctx = s->ctx;
-    OutArg o;
-    if (const int rc = stage_out(ctx, to, sizeof(double) * 3 * (size_t)s->n, stage, &o)) return rc;
+    const size_t bytes = sizeof(double) * 3 * (size_t)s->n;
+    SOFIA_CUDA(ctx, ctx->stage[stage].ensure(bytes));
+    double *from = ctx->stage[stage].as<double>();
     launch_pdl(k_state_out<T>, grid_for(3L * s->n, 256), 256, 0, ctx->stream, s->n, v[0].as<T>(),
-               v[1].as<T>(), v[2].as<T>(), (double *)o.dev);
+               v[1].as<T>(), v[2].as<T>(), from);
     SOFIA_CUDA(ctx, cudaGetLastError());
-    return finish_out(ctx, o);
+    if (!is_device_ptr(to)) return ctx->copies->out(to, from, bytes);
+    SOFIA_CUDA(ctx, cudaMemcpyAsync(to, from, bytes, cudaMemcpyDefault, ctx->stream));
+    return SOFIA_OK;
 }
 int forces_out(Sys *s, double *f) { return state_out<long long>(s, s->f, f, 2); }
 }  // namespace sofia
