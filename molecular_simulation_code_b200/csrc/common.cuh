@@ -137,10 +137,10 @@ inline int cuda_fail(sofia_nb_ctx *ctx, cudaError_t e, const char *where,
         if (_e != cudaSuccess) return sofia::cuda_fail((ctx), _e, #call, __FILE__, __LINE__); \
     } while (0)
 
-// The host copies of one call of the C ABI (transfer.cu), made at its start: in()
-// returns with the host array free to reuse, out() may deliver as late as sync(),
-// which also waits for the context's stream.  A call that fails before sync()
-// delivers nothing more.
+// The host copies of one call of the C ABI (transfer.cu), made at its start.  A
+// pageable array is free to reuse when in() returns; a pinned one is read, and out()
+// may deliver, as late as sync(), which also waits for the context's stream.  A call
+// that fails before sync() leaves no copy of a host array in flight.
 class HostCopies {
   public:
     explicit HostCopies(sofia_nb_ctx *c);
@@ -165,7 +165,7 @@ class HostCopies {
     Out outs[MAX];
     int nslot = 0, nout = 0;
     size_t used = 0;
-    bool idle = true;  // no copy of the slots is in flight
+    bool idle = true;  // no copy of the slots or of the caller's arrays is in flight
 };
 
 // True when p is device (or managed) memory; host pointers are staged.

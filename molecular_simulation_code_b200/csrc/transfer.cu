@@ -190,7 +190,9 @@ void transfer_close() {
 HostCopies::HostCopies(sofia_nb_ctx *c) : ctx(c), outer(c->copies) { c->copies = this; }
 
 HostCopies::~HostCopies() {
-    if (nslot > 0 && !idle) cudaStreamSynchronize(ctx->stream);  // a call that failed half-way
+    // a call that failed half-way: neither its slots nor the caller's pinned arrays may
+    // be in use when it returns
+    if (!idle) cudaStreamSynchronize(ctx->stream);
     for (int i = 0; i < nslot; ++i) give_slot(slots[i]);
     ctx->copies = outer;
 }
@@ -208,7 +210,6 @@ char *HostCopies::reserve(size_t bytes) {
     }
     char *p = slots[nslot - 1] + used;
     used += need;
-    idle = false;
     return p;
 }
 
@@ -224,6 +225,7 @@ int HostCopies::in(void *dev, const void *host, size_t bytes) {
             if (move_large(ctx, false, const_cast<void *>(host), dev, bytes, &rc)) return rc;
         }
     }
+    idle = false;
     SOFIA_CUDA(ctx, cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
     return SOFIA_OK;
 }
@@ -233,6 +235,7 @@ int HostCopies::out(void *host, const void *dev, size_t bytes) {
         if (bytes <= SLOT) {
             char *p = nout < MAX ? reserve(bytes) : nullptr;
             if (p) {
+                idle = false;
                 SOFIA_CUDA(ctx, cudaMemcpyAsync(p, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
                 outs[nout++] = Out{host, p, bytes};
                 return SOFIA_OK;
@@ -242,6 +245,7 @@ int HostCopies::out(void *host, const void *dev, size_t bytes) {
             if (move_large(ctx, true, host, const_cast<void *>(dev), bytes, &rc)) return rc;
         }
     }
+    idle = false;
     SOFIA_CUDA(ctx, cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     return SOFIA_OK;
 }
