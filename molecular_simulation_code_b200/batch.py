@@ -3,7 +3,8 @@
 A ``Batch`` groups device-resident systems and advances all of them together
 (``sofia_batch_md_run``): each kernel of a step runs once for every replica,
 and steps run as captured graphs of ``seg`` steps.  Members can change between
-runs (``set_systems``) without a graph recapture.  Replicas never exchange data, so each replica's
+runs (``set_systems``); the graphs are captured anew only when the amount of work
+has changed by a third or more.  Replicas never exchange data, so each replica's
 trajectory is bit-identical to the same replica run alone.
 
 ``autotune`` times short MD segments of one replica per candidate shape --
@@ -60,7 +61,7 @@ class Batch:
         return [dict(zip(MD_ENERGY_NAMES, row.tolist())) for row in e]
 
     def set_systems(self, systems: list):
-        """New members for the next run (continuous batching, no graph recapture)."""
+        """New members for the next run (continuous batching)."""
         arr = (C.c_void_p * len(systems))(*[s.handle.value for s in systems])
         self.ctx.check(self.ctx._lib.sofia_batch_set_systems(self.handle, arr, len(systems)))
         self.systems = list(systems)

@@ -1330,7 +1330,8 @@ extern "C" int sofia_system_md_forces(sofia_system *ss, int terms, double *f, do
 // bit-identical to the same replica run alone.  Steps are captured as CUDA
 // graphs of `seg` steps (100 by default); the graphs hold only the address of
 // the device table, which the host rewrites when membership changes or a list
-// grows, so neither needs a recapture.  Replicas never exchange data (the
+// grows.  A new row split or members of much more or less work get graphs of their
+// own (batch_graphs, batch_grids_fit).  Replicas never exchange data (the
 // reference runs one replica per MPI rank, Source/MD.f90:26-44).
 namespace sofia {
 namespace {
@@ -1569,6 +1570,30 @@ static void batch_step(BatchDev *tab, Sys *s0, bool energy, bool rattle, sofia_n
 
 }  // namespace sofia
 
+namespace sofia {
+// The graphs of a batch for one row split.  They hold the address of the device table,
+// so members may change under them; the split is part of their kernels, and their
+// grids are sized from the members they were captured with.
+struct BatchGraphs {
+    // [0] one step, [1] one step with energies, [2] seg steps, [3] seg steps with
+    // energies on the last
+    cudaGraphExec_t exec[4] = {nullptr, nullptr, nullptr, nullptr};
+    bool ok = false;
+    bool rattle = false;                // they hold the RATTLE launch
+    PairKey key{};                      // the pair constants they hold
+    int row_blocks = 0;                 // BK_W256 virtual blocks of the members
+    long long launches[4] = {0, 0, 0, 0};  // kernel launches each holds
+    void drop() {
+        for (auto &g : exec)
+            if (g) {
+                cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
+        ok = false;
+    }
+};
+}  // namespace sofia
+
 struct sofia_batch {
     sofia_nb_ctx *ctx = nullptr;
     std::vector<sofia_system *> sys;
@@ -1580,22 +1605,13 @@ struct sofia_batch {
     int seg = 100;                      // steps per captured segment graph
     int split = 1;                      // warps per list row of the force-only pair kernel
     int nsm = 148;
-    // captured graphs: [0] one step, [1] one step with energies, [2] seg steps,
-    // [3] seg steps with energies on the last
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
-    int graph_ok = 0;
-    int graph_rattle = 0;               // the graphs hold the RATTLE launch
-    sofia::PairKey graph_key{};         // the pair constants the graphs hold
-    long long graph_launches[4] = {0, 0, 0, 0};  // kernel launches each graph holds
+    sofia::BatchGraphs graphs[3];       // for 1, 2 and 4 warps per list row
 };
 
+static sofia::BatchGraphs &batch_graphs(sofia_batch *b) { return b->graphs[b->split >> 1]; }
+
 static void batch_drop_graphs(sofia_batch *b) {
-    for (auto &g : b->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
-    b->graph_ok = 0;
+    for (auto &g : b->graphs) g.drop();
 }
 
 static int batch_check_members(sofia_nb_ctx *ctx, sofia_system *const *systems, int n) {
@@ -1626,11 +1642,9 @@ static int batch_upload(sofia_batch *b) {
     if (b->htab.size() != sizeof(sofia::BatchDev)) b->htab.assign(sizeof(sofia::BatchDev), 0);
     auto *h = reinterpret_cast<sofia::BatchDev *>(b->htab.data());
     h->nrep = n;
-    if (!b->graph_ok) {  // the captured graphs keep the split they were captured with
-        std::vector<const Sys *> members;
-        for (auto *m : b->sys) members.push_back(&m->s);
-        b->split = sofia::batch_pair_split(members);
-    }
+    std::vector<const Sys *> members;
+    for (auto *m : b->sys) members.push_back(&m->s);
+    b->split = sofia::batch_pair_split(members);
     for (int k = 0; k < sofia::BK_N; ++k) h->pre[k][0] = 0;
     for (int r = 0; r < n; ++r) {
         Sys *s = &b->sys[r]->s;
@@ -1680,9 +1694,9 @@ extern "C" int sofia_batch_destroy(sofia_batch *b) {
     return SOFIA_OK;
 }
 
-// Replaces the batch's members (continuous batching).  The captured graphs stay
-// valid when the new members share the first member's pair constants and need
-// no RATTLE launch the graphs lack.
+// Replaces the batch's members (continuous batching).  Captured graphs stay valid
+// when the new members share the pair constants they hold and need no RATTLE launch
+// that they lack; the next run takes the ones of the new members' row split.
 extern "C" int sofia_batch_set_systems(sofia_batch *b, sofia_system *const *systems, int n) {
     if (!b || !systems) return SOFIA_EINVAL;
     sofia_nb_ctx *ctx = b->ctx;
@@ -1691,12 +1705,10 @@ extern "C" int sofia_batch_set_systems(sofia_batch *b, sofia_system *const *syst
     if (rc) return rc;
     SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     b->sys.assign(systems, systems + n);
-    if (b->graph_ok) {
-        bool rat = false;
-        for (auto *s : b->sys) rat = rat || (s->s.md.rattle && s->s.md.nshake);
-        const bool keep = (!rat || b->graph_rattle) && b->graph_key == sofia::pair_key(&b->sys[0]->s);
-        if (!keep) batch_drop_graphs(b);
-    }
+    bool rat = false;
+    for (auto *s : b->sys) rat = rat || (s->s.md.rattle && s->s.md.nshake);
+    for (auto &g : b->graphs)
+        if (g.ok && ((rat && !g.rattle) || !(g.key == sofia::pair_key(&b->sys[0]->s)))) g.drop();
     return SOFIA_OK;
 }
 
@@ -1711,8 +1723,10 @@ extern "C" int sofia_batch_set_segment(sofia_batch *b, int steps) {
     return SOFIA_OK;
 }
 
+// Captures the graphs of the members' row split.
 static int batch_capture(sofia_batch *b) {
-    batch_drop_graphs(b);
+    sofia::BatchGraphs &bg = batch_graphs(b);
+    bg.drop();
     sofia_nb_ctx *ctx = b->ctx;
     SOFIA_CUDA(ctx, sofia::side_open(ctx));
     cudaStream_t ms = ctx->stream;
@@ -1737,7 +1751,7 @@ static int batch_capture(sofia_batch *b) {
         }
         cudaError_t ce = cudaStreamEndCapture(ms, &graph);
         if (ce != cudaSuccess) return sofia::cuda_fail(ctx, ce, "cudaStreamEndCapture (batch)");
-        ce = cudaGraphInstantiate(&b->graph[g], graph, 0);
+        ce = cudaGraphInstantiate(&bg.exec[g], graph, 0);
         cudaGraphDestroy(graph);
         if (ce != cudaSuccess) return sofia::cuda_fail(ctx, ce, "cudaGraphInstantiate (batch)");
     }
@@ -1746,14 +1760,25 @@ static int batch_capture(sofia_batch *b) {
     // kicks are chained; energies add the two pair-energy and four MD-energy
     // reductions
     const long long body = 1 + 9 + 2, closing = 1 + (rat ? 1 : 0);
-    b->graph_launches[0] = body + closing;
-    b->graph_launches[1] = body + closing + 6;
-    b->graph_launches[2] = rat ? b->seg * (body + closing) : b->seg * body + closing;
-    b->graph_launches[3] = b->graph_launches[2] + 6;
-    b->graph_rattle = rat;
-    b->graph_key = sofia::pair_key(s0);
-    b->graph_ok = 1;
+    bg.launches[0] = body + closing;
+    bg.launches[1] = body + closing + 6;
+    bg.launches[2] = rat ? b->seg * (body + closing) : b->seg * body + closing;
+    bg.launches[3] = bg.launches[2] + 6;
+    bg.rattle = rat;
+    bg.key = sofia::pair_key(s0);
+    bg.row_blocks = row_blocks;
+    bg.ok = true;
     return SOFIA_OK;
+}
+
+// Whether graphs captured with members of `held` row blocks serve members of `rows`.
+// Their grids cover any number of rows, but short grids make blocks walk several rows
+// one after the other and long ones launch blocks for nothing (us per step of 16 and 64
+// replicas with graphs captured at 0.5 / 0.7 / 1 / 2.3 / 4.5 times their rows: 505 /
+// 488 / 487 / 491 / 507 and 1,918 / 1,899 / 1,901 / - / -; 8,000 for 64 replicas with
+// those of one replica and its 4 warps per row).
+static bool batch_grids_fit(int held, int rows) {
+    return 3L * rows <= 4L * held && 2L * rows >= held;
 }
 
 // Runs nsteps steps of every replica: segments of `seg` steps as one graph
@@ -1794,7 +1819,9 @@ extern "C" int sofia_batch_md_run(sofia_batch *b, int nsteps, int energy_every,
                 SOFIA_CUDA(ctx, cudaStreamSynchronize(s->ctx->stream));
             }
         }
-        if (!b->graph_ok) {
+        sofia::BatchGraphs &bg = batch_graphs(b);
+        const auto *h = reinterpret_cast<const sofia::BatchDev *>(b->htab.data());
+        if (!bg.ok || !batch_grids_fit(bg.row_blocks, h->pre[sofia::BK_W256][n])) {
             rc = batch_capture(b);
             if (rc) return rc;
         }
@@ -1804,8 +1831,8 @@ extern "C" int sofia_batch_md_run(sofia_batch *b, int nsteps, int energy_every,
             const bool full = left >= b->seg;
             const int k = full ? b->seg : 1;
             const bool en = want_e && left == k;
-            SOFIA_CUDA(ctx, cudaGraphLaunch(b->graph[(full ? 2 : 0) + (en ? 1 : 0)], ms));
-            launched += b->graph_launches[(full ? 2 : 0) + (en ? 1 : 0)];
+            SOFIA_CUDA(ctx, cudaGraphLaunch(bg.exec[(full ? 2 : 0) + (en ? 1 : 0)], ms));
+            launched += bg.launches[(full ? 2 : 0) + (en ? 1 : 0)];
             left -= k;
         }
         SOFIA_CUDA(ctx, sofia::launch_pdl(sofia::k_status_b, b->nsm, 32, 0, ms, tab,

@@ -249,7 +249,7 @@ struct BatchDev {
 // virtual blocks b, b + gridDim.x, ...  The pair, search and prune kernels are
 // launched with one block per virtual block of all members at capture time, so
 // each block takes at most one and the hardware block scheduler balances the
-// uneven rows; members added later without a recapture are covered by the
+// uneven rows; members added later under the same graphs are covered by the
 // stride.  ACTIVE_LOOP walks the kind-KIND blocks of the replicas active for
 // trigger mask M (BatchActive).  Inside, d is the replica's entry and lb the
 // block index within that replica.

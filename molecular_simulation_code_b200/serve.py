@@ -16,8 +16,7 @@ runs many such segments at once on one GPU:
 * all running replicas advance together in one ``Batch`` (every kernel of a
   step once for all of them, captured segment graphs); requests that arrive
   meanwhile join at the next chunk boundary and finished ones leave, by
-  changing the batch's members without a graph recapture (continuous
-  batching);
+  changing the batch's members (continuous batching);
 * a new replica's damped warm-in from its lattice start runs inside the batch
   (1 fs steps, strong friction) instead of blocking the running replicas;
 * a finished segment ends with the largest-cluster analysis on the device-
