@@ -152,19 +152,19 @@ class HostCopies {
     int sync();
 
   private:
-    static constexpr int MAX = 16;
+    static constexpr int MAX = 16, MAX_OUT = 64;
     struct Out {
         void *host;
         const char *pinned;
         size_t bytes;
     };
-    char *reserve(size_t bytes);
+    char *reserve(size_t *bytes);
     sofia_nb_ctx *ctx;
     HostCopies *outer;  // of a call that this one is part of
     char *slots[MAX];
-    Out outs[MAX];
+    Out outs[MAX_OUT];
     int nslot = 0, nout = 0;
-    size_t used = 0;
+    size_t used[MAX];
     bool idle = true;  // no copy of the slots or of the caller's arrays is in flight
 };
 

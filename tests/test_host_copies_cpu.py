@@ -2,7 +2,7 @@
 for the CUDA runtime in which a queued copy runs as late as the real one may: when its
 stream or event is waited for.  Covers what a call leaves behind when it fails half-way,
 arrays that are reused at once, every size class in both directions, a call that finds all
-pinned slots taken, and the slots' return with the last context."""
+pinned slots taken, what a first call pins, and the slots' return with the last context."""
 import os
 import shutil
 import subprocess
@@ -15,6 +15,7 @@ CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include
 SRC = r"""
 #include <cmath>
 #include "transfer.cu"
+#include <atomic>
 #include <cstdlib>
 #include <deque>
 #include <functional>
@@ -28,7 +29,7 @@ static std::map<cudaStream_t, std::deque<std::function<void()>>> g_q;
 static std::map<char *, size_t> g_pinned;      // cudaHostAlloc and the caller's pinned arrays
 static std::map<cudaEvent_t, cudaStream_t> g_ev;
 static size_t g_alloc = 0, g_bytes = 0, g_most = 0;  // live cudaHostAlloc blocks
-static long g_id = 100;
+static std::atomic<long> g_id{100};
 static bool pinned_(const void *p) {
     auto it = g_pinned.upper_bound((char *)p);
     return it != g_pinned.begin() && (char *)p < (--it)->first + it->second;
@@ -108,7 +109,7 @@ struct Ctx : sofia_nb_ctx {
     ~Ctx() { sofia::transfer_close(); }
 };
 static const size_t SIZES[] = {1, 255, 256, 65536, 65537, 200000, 262143, 262144, 262145, 700001,
-                               1048576, 1048577, 2097153, 9000001};
+                               1048576, 1048577, 2097153, 9000001, 16777216, 20000003};
 // one array in and back: reused as soon as in() returns, delivered by sync()
 static void round_trip(sofia_nb_ctx *c, size_t n, unsigned seed) {
     const Bytes want = noise(n, seed);
@@ -176,6 +177,19 @@ static void slots_taken() {
     for (size_t k = 0; k < a.size(); ++k) CHECK(dev[k] == a[k]);
     CHECK(g_most <= (16u << 20));
 }
+// What a new context pins: a large array, or a call's small ones, fit in the 2 MB that the
+// driver pins at least, beside the context's own few words.
+static void first_use() {
+    const size_t most = 7u << 18;
+    { Ctx c; round_trip(&c, 9000000, 5); CHECK(g_most <= most); }
+    { Ctx c; round_trip(&c, 216000, 6); CHECK(g_most <= most); }
+    Ctx c;
+    Bytes a = noise(540000, 8), dev(540000);
+    sofia::HostCopies h(&c);
+    for (size_t n : {384000, 96000, 540000, 288000}) CHECK(h.in(dev.data(), a.data(), n) == SOFIA_OK);
+    CHECK(h.out(a.data(), dev.data(), 288000) == SOFIA_OK);
+    CHECK(h.sync() == SOFIA_OK && g_most <= most);
+}
 static void threads() {
     auto work = [](unsigned seed) {
         for (int k = 0; k < 20; ++k) {
@@ -192,6 +206,7 @@ int main(int argc, char **argv) {
     if (what == "sizes") sizes();
     if (what == "slots_taken") slots_taken();
     if (what == "threads") threads();
+    if (what == "first_use") first_use();
     CHECK(g_alloc == 0 && pending() == 0);  // the last context took the slots with it
     printf(failures ? "failed\n" : "ok\n");
     return failures != 0;
@@ -212,7 +227,8 @@ def harness(tmp_path_factory):
     return str(d / "copies")
 
 
-@pytest.mark.parametrize("what", ["failed_calls", "sizes", "slots_taken", "threads"])
+@pytest.mark.parametrize("what", ["failed_calls", "sizes", "slots_taken", "threads",
+                                  "first_use"])
 def test_host_copies(harness, what):
     r = subprocess.run([harness, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
