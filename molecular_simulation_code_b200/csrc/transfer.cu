@@ -20,7 +20,6 @@
 // slot tell (BIG_FROM: the 37 MB list of 9,000 atoms there and back 6.6 ms a pass in
 // slots of 256 KB, 4.8 in 1 MB) take big slots.
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 #include "common.cuh"
@@ -177,7 +176,7 @@ bool move_large(sofia_nb_ctx *ctx, bool out, void *host, void *dev, size_t bytes
         for (int t = 1; t < got; ++t) {
             try {
                 th[t] = std::thread(move_share, &w[t]);
-            } catch (const std::system_error &) {
+            } catch (...) {  // no thread, or no memory for one
                 move_share(&w[t]);
             }
         }

@@ -2,7 +2,8 @@
 for the CUDA runtime in which a queued copy runs as late as the real one may: when its
 stream or event is waited for.  Covers what a call leaves behind when it fails half-way,
 arrays that are reused at once, every size class in both directions, a call that finds all
-pinned slots taken, what a first call pins, and the slots' return with the last context."""
+pinned slots taken, threads that cannot be made, what a first call pins, and the slots'
+return with the last context."""
 import os
 import shutil
 import subprocess
@@ -47,7 +48,21 @@ static size_t pending() {
     for (auto &q : g_q) n += q.second.size();
     return n;
 }
-#define LOCK std::lock_guard<std::recursive_mutex> lk(g_m)
+// operator new fails for this thread, outside the stand-ins
+static thread_local bool t_nomem = false;
+struct Exempt {
+    bool was = t_nomem;
+    Exempt() { t_nomem = false; }
+    ~Exempt() { t_nomem = was; }
+};
+void *operator new(size_t n) {
+    void *p = t_nomem ? nullptr : malloc(n);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
+#define LOCK Exempt ex; std::lock_guard<std::recursive_mutex> lk(g_m)
 extern "C" {
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
     LOCK; *p = malloc(n); g_pinned[(char *)*p] = n; ++g_alloc; g_bytes += n;
@@ -200,6 +215,18 @@ static void threads() {
     std::thread t1(work, 1000), t2(work, 2000), t3(work, 3000);
     t1.join(); t2.join(); t3.join();
 }
+// Threads that cannot be made: the calling one moves their shares.
+static void no_memory() {
+    Ctx c;
+    const Bytes want = noise(9000001, 9);
+    Bytes dev(want.size()), got(want.size());
+    sofia::HostCopies h(&c);
+    t_nomem = true;
+    const int in = h.in(dev.data(), want.data(), want.size());
+    const int out = h.out(got.data(), dev.data(), got.size());
+    t_nomem = false;
+    CHECK(in == SOFIA_OK && out == SOFIA_OK && h.sync() == SOFIA_OK && got == want);
+}
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "failed_calls") failed_calls();
@@ -207,6 +234,7 @@ int main(int argc, char **argv) {
     if (what == "slots_taken") slots_taken();
     if (what == "threads") threads();
     if (what == "first_use") first_use();
+    if (what == "no_memory") no_memory();
     CHECK(g_alloc == 0 && pending() == 0);  // the last context took the slots with it
     printf(failures ? "failed\n" : "ok\n");
     return failures != 0;
@@ -228,7 +256,7 @@ def harness(tmp_path_factory):
 
 
 @pytest.mark.parametrize("what", ["failed_calls", "sizes", "slots_taken", "threads",
-                                  "first_use"])
+                                  "first_use", "no_memory"])
 def test_host_copies(harness, what):
     r = subprocess.run([harness, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
