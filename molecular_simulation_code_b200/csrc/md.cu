@@ -882,9 +882,11 @@ static int md_forces(Sys *s, bool energy, bool force_build, bool disp_done = fal
         // A step: the forces were cleared with the kick, so the bonded terms need the
         // new positions only and run beside the list maintenance and the pair kernel;
         // the force unpack adds to their sums.  Their 10 us of latency at 9,000 atoms
-        // hide behind kernels that leave most of the GPU idle (a step 58.1 -> 51.8 us,
-        // at 37,000 atoms 120.8 -> 115.6); at 275,000 atoms the two compete and the step
-        // takes as long as before (585 and 587).
+        // hide behind kernels that leave most of the GPU idle (a step 58.1 -> 51.8 us).
+        // Every size takes this form: with the terms after the pair kernel instead,
+        // 37,000 / 55,000 / 90,000 / 145,000 / 275,000 atoms take 117.4 / 153.3 / 217.2 /
+        // 320.0 / 573.5 us, against 113.4 / 148.9 / 215.4 / 318.9 / 573.8 (runs differ by
+        // 0.5), and in FP64 208.1 / 283.8 / 440.0 against 203.5 / 278.8 / 437.7.
         sofia_nb_ctx *ctx = s->ctx;
         if (nterm > 0) {
             SOFIA_CUDA(ctx, side_open(ctx));
@@ -1756,9 +1758,9 @@ static int batch_capture(sofia_batch *b) {
         if (ce != cudaSuccess) return sofia::cuda_fail(ctx, ce, "cudaGraphInstantiate (batch)");
     }
     // a step: kick+drift, the pair path (active-replica compaction, bin, scan, sort,
-    // pack with the cluster boxes, search, prune, pair, unpack), bonded, SHAKE; then the closing kick (+ RATTLE), once per segment when the
-    // kicks are chained; energies add the two pair-energy and four MD-energy
-    // reductions
+    // pack with the cluster boxes, search, prune, pair, unpack), bonded, SHAKE; then
+    // the closing kick (+ RATTLE), once per segment when the kicks are chained;
+    // energies add the two pair-energy and four MD-energy reductions
     const long long body = 1 + 9 + 2, closing = 1 + (rat ? 1 : 0);
     bg.launches[0] = body + closing;
     bg.launches[1] = body + closing + 6;

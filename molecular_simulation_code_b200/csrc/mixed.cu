@@ -1221,13 +1221,13 @@ inline cudaError_t pair_smem_optin(int nt) {
     return e;
 }
 
-// Slot-ordered fixed-point pair forces -> the caller's atom order (sets the
-// force arrays; bonded terms add to them afterwards).  Flags sums outside the
-// fixed-point range.
+// Slot-ordered fixed-point pair forces -> the caller's atom order.  In an MD step
+// (ADD) the bonded terms have been summed in the force arrays already and the pair
+// forces are added to them; otherwise they are set, and bonded terms add afterwards.
+// Flags sums outside the fixed-point range.
 // With flag != NULL, thread 0 also counts this step's list build and prune in
 // cnt and clears the trigger word for the next step's displacement check (only
-// bits are ORed into it).  With lg.on, each atom's Langevin force is added.  ADD: onto
-// what the force arrays hold.
+// bits are ORed into it).  With lg.on, each atom's Langevin force is added.
 // One thread per atom: the slot forces are the only scattered reads, where a thread per
 // slot scattered the force arrays' reads and writes and the thermostat's inputs (MD step
 // at 275,000 atoms 582 -> 577 us, at 9,000 49.4 -> 48.7).

@@ -2,9 +2,12 @@
 // LJ + DSF pair kernel, 1-4 pairs and exclusion corrections.
 //
 // This translation unit is compiled with -fmad=false: every real*4 and real*8
-// operation is rounded on its own, in the Fortran evaluation order, so the
-// neighbour sets are bit-identical to the reference and the FP64 sums agree to
-// the last bits up to summation order.
+// operation is rounded on its own, and in the Fortran evaluation order, so the
+// neighbour sets are bit-identical to the reference.  Two forms differ in the last
+// bits: k_force_ref takes 1/r, 1/r^2 and r from one reciprocal square root instead of
+// a square root and three divisions, and sums are in another order.  Its errors
+// against 64-bit references are those of the divisions (forces within two ulps of the
+// largest, energies within 1e-10).
 //
 // Layout in HBM: positions as float4 {x,y,z,type-bits} (the reference's 16 B
 // ainfo record, loaded with one 128-bit access), cell-sorted copies for the
@@ -992,7 +995,11 @@ int check_status(sofia_nb_ctx *ctx) {
 // Atoms per warp of the list build: a chunk's sweep over 3,600 candidates is one serial
 // chain, so a system whose chunks of 8 leave warps idle takes chunks of 4 (list plus FP64
 // forces at 3,300 / 9,000 / 15,900 atoms: 199 / 247 / 274 us with 8, 165 / 226 / 297 us
-// with 4).
+// with 4).  What chunks of 4 gain is the longer sweep's, in grids of 3 and 4 cells per
+// side, where the image is taken per pair (list alone, us, 4 / 8): cut-off 10 A, 5,500
+// and 11,400 atoms 168 / 192 and 192 / 218, 16,000 168 / 146; 12 A, 9,000 and 12,500
+// atoms 244 / 284 and 208 / 236, 16,000 313 / 295; with shorter cut-offs and more cells
+// the two are within 4 %, but for 8 A at 9,000 atoms (105 / 95).
 int list_atoms(int np) { return np < 12000 ? 4 : 8; }
 
 // Bin + sort shared by sofia_cell_sort and sofia_neighbor_build.  list: the sorted
