@@ -129,7 +129,7 @@ def bench_serve(args):
         stats["cluster_sizes_seeded"] = sorted(int(r.cluster_size) for r in seeded)
         stats["cluster_sizes_top5_other"] = sorted(int(r.cluster_size) for r in srv.results
                                                    if r not in seeded)[-5:]
-        stats["batch_graph_captures"] = srv.recaptures
+        stats["batches_created"] = srv.recaptures
         stats["cluster_criterion"] = {"mrcut_A": srv.mrcut, "denscut_A": srv.denscut,
                                       "densmin": srv.densmin}
         out[name] = stats

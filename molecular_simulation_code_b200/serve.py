@@ -124,7 +124,7 @@ class Server:
         self.atom_steps = 0
         self.replica_steps = 0
         self.bytes_per_atom = float(BYTES_PER_ATOM)
-        self.recaptures = 0
+        self.recaptures = 0  # batches created
 
     # -- clock and memory -------------------------------------------------
     def now(self) -> float:
