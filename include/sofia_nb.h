@@ -442,10 +442,10 @@ int sofia_system_md_forces(sofia_system *sys, int terms, double *f, double *ener
  *       (may be NULL) receive each replica's energies of the last step when
  *       energy_every > 0 (only that step computes them).
  *   sofia_batch_set_systems: new members for the next run (continuous
- *       batching); captured graphs are kept when the new members share the
- *       pair constants, and the next run captures anew only for a row split
- *       that the batch has not run yet or when the members' list rows have
- *       left 0.5 to 1.33 times those it was captured with.
+ *       batching).  A run takes the graphs captured earlier; it captures anew
+ *       for a row split that the batch has not run yet, when the members' list
+ *       rows have left 0.5 to 1.33 times those of the capture, and when their
+ *       pair constants or RATTLE stage differ from it.
  *   sofia_batch_set_segment: steps per captured graph (1..1000).
  */
 typedef struct sofia_batch sofia_batch;

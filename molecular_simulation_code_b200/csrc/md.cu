@@ -1333,7 +1333,7 @@ extern "C" int sofia_system_md_forces(sofia_system *ss, int terms, double *f, do
 // graphs of `seg` steps (100 by default); the graphs hold only the address of
 // the device table, which the host rewrites when membership changes or a list
 // grows.  A new row split or members of much more or less work get graphs of their
-// own (batch_graphs, batch_grids_fit).  Replicas never exchange data (the
+// own (batch_graphs, batch_graphs_fit).  Replicas never exchange data (the
 // reference runs one replica per MPI rank, Source/MD.f90:26-44).
 namespace sofia {
 namespace {
@@ -1696,9 +1696,8 @@ extern "C" int sofia_batch_destroy(sofia_batch *b) {
     return SOFIA_OK;
 }
 
-// Replaces the batch's members (continuous batching).  Captured graphs stay valid
-// when the new members share the pair constants they hold and need no RATTLE launch
-// that they lack; the next run takes the ones of the new members' row split.
+// Replaces the batch's members (continuous batching).  The next run takes the graphs
+// of the new members' row split, if they fit (batch_graphs_fit).
 extern "C" int sofia_batch_set_systems(sofia_batch *b, sofia_system *const *systems, int n) {
     if (!b || !systems) return SOFIA_EINVAL;
     sofia_nb_ctx *ctx = b->ctx;
@@ -1707,10 +1706,6 @@ extern "C" int sofia_batch_set_systems(sofia_batch *b, sofia_system *const *syst
     if (rc) return rc;
     SOFIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     b->sys.assign(systems, systems + n);
-    bool rat = false;
-    for (auto *s : b->sys) rat = rat || (s->s.md.rattle && s->s.md.nshake);
-    for (auto &g : b->graphs)
-        if (g.ok && ((rat && !g.rattle) || !(g.key == sofia::pair_key(&b->sys[0]->s)))) g.drop();
     return SOFIA_OK;
 }
 
@@ -1773,14 +1768,18 @@ static int batch_capture(sofia_batch *b) {
     return SOFIA_OK;
 }
 
-// Whether graphs captured with members of `held` row blocks serve members of `rows`.
-// Their grids cover any number of rows, but short grids make blocks walk several rows
-// one after the other and long ones launch blocks for nothing (us per step of 16 and 64
-// replicas with graphs captured at 0.5 / 0.7 / 1 / 2.3 / 4.5 times their rows: 505 /
-// 488 / 487 / 491 / 507 and 1,918 / 1,899 / 1,901 / - / -; 8,000 for 64 replicas with
-// those of one replica and its 4 warps per row).
-static bool batch_grids_fit(int held, int rows) {
-    return 3L * rows <= 4L * held && 2L * rows >= held;
+// Whether graphs serve the members: these have the pair constants that the graphs hold
+// and no RATTLE stage that the graphs lack (both may change by sofia_system_md_setup),
+// and their rows fit the grids.  Grids cover any number of rows, but short ones make
+// blocks walk several rows one after the other and long ones launch blocks for nothing
+// (us per step of 16 and 64 replicas with graphs captured at 0.5 / 0.7 / 1 / 2.3 / 4.5
+// times their rows: 505 / 488 / 487 / 491 / 507 and 1,918 / 1,899 / 1,901 / - / -; 8,000
+// for 64 replicas with those of one replica and its 4 warps per row).
+static bool batch_graphs_fit(const sofia::BatchGraphs &g, const sofia_batch *b, int rows) {
+    bool rat = false;
+    for (auto *s : b->sys) rat = rat || (s->s.md.rattle && s->s.md.nshake);
+    return g.ok && g.key == sofia::pair_key(&b->sys[0]->s) && (g.rattle || !rat) &&
+           3L * rows <= 4L * g.row_blocks && 2L * rows >= g.row_blocks;
 }
 
 // Runs nsteps steps of every replica: segments of `seg` steps as one graph
@@ -1794,6 +1793,8 @@ extern "C" int sofia_batch_md_run(sofia_batch *b, int nsteps, int energy_every,
     SOFIA_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t ms = ctx->stream;
     const int n = (int)b->sys.size();
+    // members may have been set up anew since they joined
+    if (const int rc = batch_check_members(ctx, b->sys.data(), n)) return rc;
     const bool want_e = energy_every > 0 && nsteps > 0;
     SOFIA_CUDA(ctx, b->stat.ensure(sizeof(int) * sofia::ST_NSLOTS * sofia::MAXREP));
     SOFIA_CUDA(ctx, b->estat.ensure(sizeof(double) * 16 * sofia::MAXREP));
@@ -1823,7 +1824,7 @@ extern "C" int sofia_batch_md_run(sofia_batch *b, int nsteps, int energy_every,
         }
         sofia::BatchGraphs &bg = batch_graphs(b);
         const auto *h = reinterpret_cast<const sofia::BatchDev *>(b->htab.data());
-        if (!bg.ok || !batch_grids_fit(bg.row_blocks, h->pre[sofia::BK_W256][n])) {
+        if (!batch_graphs_fit(bg, b, h->pre[sofia::BK_W256][n])) {
             rc = batch_capture(b);
             if (rc) return rc;
         }
